@@ -1053,6 +1053,98 @@ __global__ void __launch_bounds__(kVarThreads, 4) k_variation(Shape s, const Dev
                dst.objidx + (size_t)out_slot * 2 * s.M, tid, nth);
 }
 
+// Codon ids between the caller's contiguous rows of L bytes and the engine's rows of Lp
+// (L rounded up to 16).  A pitched copy between the host and the device moves pageable
+// host memory row by row, so the host copies are contiguous and these two kernels
+// change the pitch on the device: a thread owns 16 bytes of the destination, read as
+// one or two aligned 16-byte pieces and shifted into place.
+
+// 16 bytes from the pieces at p[0] and, when they reach into it, p[1] (off: 0 .. 15)
+__device__ __forceinline__ uint4 shifted_piece(const uint4 *__restrict__ p, int off, bool second)
+{
+    const uint4 x = p[0], y = second ? p[1] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    uint32_t u[7], r[5];
+#pragma unroll
+    for (int i = 0; i < 7; i++) u[i] = off & 4 ? v[i + 1] : v[i];
+#pragma unroll
+    for (int i = 0; i < 5; i++) r[i] = off & 8 ? u[i + 2] : u[i];
+    const int b = 8 * (off & 3);
+    return make_uint4(__funnelshift_r(r[0], r[1], b), __funnelshift_r(r[1], r[2], b), __funnelshift_r(r[2], r[3], b),
+                      __funnelshift_r(r[3], r[4], b));
+}
+
+// packed: rows x L bytes, 16-byte aligned, readable up to the next multiple of 16;
+// ids: rows x Lp, zero past L.  *bad takes the index of the first id >= 64.
+__global__ void __launch_bounds__(256) k_unpack_rows(const uint8_t *__restrict__ packed, size_t rows, int L, int Lp,
+                                                     uint8_t *__restrict__ ids, unsigned long long *bad)
+{
+    const int per = Lp >> 4;
+    const size_t total = rows * per;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const size_t row = e / per;
+        const int c = (int)(e - row * per) * 16, live = min(16, L - c);
+        const size_t at = row * L + c;
+        const int off = (int)(at & 15);
+        uint4 v = shifted_piece(reinterpret_cast<const uint4 *>(packed + (at - off)), off, off + live > 16);
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {  // clear the bytes past the row's end
+            const int k = live - 4 * i;
+            if (k < 4) w[i] &= k <= 0 ? 0u : (1u << (8 * k)) - 1u;
+        }
+        if ((w[0] | w[1] | w[2] | w[3]) & 0xc0c0c0c0u) {
+            int k = 0;
+            while (!((w[k >> 2] >> (8 * (k & 3))) & 0xc0u)) k++;
+            atomicMin(bad, (unsigned long long)(at + k));
+        }
+        reinterpret_cast<uint4 *>(ids)[e] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// the way back: packed must be 16-byte aligned and is written up to rows * L exactly
+__global__ void __launch_bounds__(256) k_pack_rows(const uint8_t *__restrict__ ids, size_t rows, int L, int Lp,
+                                                   uint8_t *__restrict__ packed)
+{
+    const size_t bytes = rows * L, total = (bytes + 15) / 16;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const size_t at = 16 * e;
+        size_t row = at / L;
+        int c = (int)(at - row * L);
+        if (c + 16 <= L) {  // inside one row, whose pitch covers the second piece
+            const int off = c & 15;
+            reinterpret_cast<uint4 *>(packed)[e] =
+                shifted_piece(reinterpret_cast<const uint4 *>(ids + row * Lp + (c - off)), off, off != 0);
+            continue;
+        }
+        const int live = bytes - at < 16 ? (int)(bytes - at) : 16;
+        for (int k = 0; k < live; k++) {
+            packed[at + k] = ids[row * Lp + c];
+            if (++c == L) {
+                c = 0;
+                row++;
+            }
+        }
+    }
+}
+
+static int row_blocks(size_t pieces) { return (int)std::min<size_t>((pieces + 255) / 256, 148 * 16); }
+
+cudaError_t launch_unpack_rows(const uint8_t *packed, size_t rows, int L, int Lp, uint8_t *ids, unsigned long long *bad,
+                               cudaStream_t st)
+{
+    if (rows == 0) return cudaSuccess;
+    k_unpack_rows<<<row_blocks(rows * (Lp >> 4)), 256, 0, st>>>(packed, rows, L, Lp, ids, bad);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack_rows(const uint8_t *ids, size_t rows, int L, int Lp, uint8_t *packed, cudaStream_t st)
+{
+    if (rows == 0) return cudaSuccess;
+    k_pack_rows<<<row_blocks((rows * L + 15) / 16), 256, 0, st>>>(ids, rows, L, Lp, packed);
+    return cudaGetLastError();
+}
+
 size_t var_smem_bytes(const Shape &s)
 {
     return ((sizeof(VarSmem) + 15) & ~size_t(15)) + (size_t)s.m * s.Lp + (size_t)s.m * s.Wp * sizeof(uint2) +
