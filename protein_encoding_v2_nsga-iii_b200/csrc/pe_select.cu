@@ -924,86 +924,189 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(Shape s, const float 
     if (tid == 0) sc.info[5] = rc - last_size;
 }
 
-// reference points staged in k_assoc's shared memory up to this size (larger sets are
-// read from global memory, so the CTAs stay small)
-constexpr size_t kAssocSmemMax = 16 * 1024;
+// referenceBasedSorting phase 1 (:1105-1180) on the whole grid: the perpendicular
+// distance of every solution of fronts 0..last to its nearest reference point
+// (include/utils.cuh:1149-1171), lowest index on ties.
+//
+// The distance of one pair takes two roundings that matter for time, a correctly
+// rounded division and a square root, and R of them per solution made this kernel
+// issue-bound at large R.  Only the nearest point's distance is kept, so the others
+// are ruled out first: with u = w / |w|, the squared distance of f to the line of w is
+// F - s^2, s = u . f and F = f . f, so the nearest point has the largest s^2.  A warp
+// takes SOLS solutions, its lanes the points, and finds the largest s^2 (MM
+// multiply-adds a pair; a point read from shared memory serves the SOLS solutions);
+// a second pass over the points evaluates the reference's own formula, operation by
+// operation, for those whose s^2 comes within kAssocSlack * F of it.  Which points that
+// leaves cannot change the result: s^2 is off by less than 1e-6 F (MM products and the
+// rounded u), the reference's rounded squared distance by less than 2e-6 F (its
+// residuals are each off by at most (MM + 3) 2^-24 |f|), and equal distances after the
+// square root differ by less than 2.4e-7 of the squared ones; all together below a
+// third of the slack.  Where F is not inside 1e-30 .. 1e30 (overflow, subnormals,
+// infinities, NaN) every point is evaluated; a point of NaN s is too.
+// Measured: 36.8 us for 8192 solutions and 4060 points of four objectives (the whole
+// selection call 488 -> 471 us), 5.9 us for 2048 solutions and 165 points (was 6.8).
+constexpr float kAssocSlack = 2e-5f;
+// points (normalised, MM padded to 4 or 8 floats) in shared memory up to this size; a
+// larger set is taken in chunks that are staged again for the second pass
+constexpr size_t kAssocSmemMax = 96 * 1024;
+__host__ __device__ constexpr int assoc_pad(int M) { return M <= 4 ? 4 : 8; }
+__host__ __device__ inline int assoc_chunk(int R, int M)
+{
+    const int most = (int)(kAssocSmemMax / (sizeof(float) * assoc_pad(M)));
+    return R < most ? R : most;
+}
 
-// referenceBasedSorting phase 1 (:1105-1180) on the whole grid: one warp per
-// solution of fronts 0..last, lanes over reference points; perpendicular
-// distance (include/utils.cuh:1149-1171), argmin with the lowest index on ties.
-// MM: the objective count when known at compile time (0: s.M at run time)
-template <int MM>
+// the reference's perpendicular distance of f to reference point w
+template <int MM> __device__ __forceinline__ float assoc_distance(const float (&f)[MM], const float *__restrict__ w)
+{
+    float num = 0.0f, den = 0.0f, wk[MM];
+#pragma unroll
+    for (int k = 0; k < MM; k++) {
+        wk[k] = __ldg(w + k);
+        num = __fadd_rn(num, __fmul_rn(wk[k], f[k]));
+        den = __fadd_rn(den, __fmul_rn(wk[k], wk[k]));
+    }
+    const float kk = __fdiv_rn(num, den);
+    float d2 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < MM; k++) {
+        const float e = __fsub_rn(__fmul_rn(kk, wk[k]), f[k]);
+        d2 = __fadd_rn(d2, __fmul_rn(e, e));
+    }
+    return __fsqrt_rn(d2);
+}
+
+template <int MM, int SOLS>
 __global__ void __launch_bounds__(256) k_assoc(Shape s, const float *__restrict__ obj,
                                                const float *__restrict__ refpts, SelectScratch sc)
 {
     if (sc.info[3]) return;  // fronts filled N exactly: no niching (uniform over the grid)
-    const int M = MM > 0 ? MM : s.M, R = s.R;
-    constexpr int KU = MM > 0 ? MM : kMaxObj;  // unrolled loop bound (k < M guards the rest)
-    const int rc = sc.info[0], count0 = sc.info[5];
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    float ideal[kMaxObj], span[kMaxObj];
+    constexpr int PAD = assoc_pad(MM);
+    const int R = s.R, rc = sc.info[0], count0 = sc.info[5];
+    const int lane = threadIdx.x & 31, t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * SOLS;
+    if (blockIdx.x * 8 * SOLS >= rc) return;  // uniform over the CTA
+    extern __shared__ __align__(16) float un[];  // [chunk][PAD] normalised points
+    const int chunk = assoc_chunk(R, MM);
+    auto stage = [&](int j0) {
+        const int nc = min(chunk, R - j0);
+        for (int j = threadIdx.x; j < nc; j += 256) {
+            float w[PAD] = {};
+            float den = 0.0f;
 #pragma unroll
-    for (int k = 0; k < KU; k++) {
-        if (k >= M) break;
-        ideal[k] = sc.finfo[k];
-        span[k] = __fsub_rn(sc.finfo[2 * M + k], ideal[k]);
-    }
-    // the reference points in shared memory when they fit (every warp of the CTA reads them)
-    extern __shared__ __align__(16) float rsm[];
-    const bool staged = (size_t)R * M * sizeof(float) <= kAssocSmemMax;
-    if (staged)
-        for (int e = threadIdx.x; e < R * M; e += blockDim.x) rsm[e] = refpts[e];
-    __syncthreads();
-    const float *rp = staged ? rsm : refpts;
-    for (int t = gw; t < rc; t += nw) {
-        const int sol = sc.sorted[t];
-        float f[kMaxObj];
+            for (int k = 0; k < MM; k++) {
+                w[k] = __ldg(refpts + (size_t)(j0 + j) * MM + k);
+                den = fmaf(w[k], w[k], den);
+            }
+            const float r = rsqrtf(den);
 #pragma unroll
-        for (int k = 0; k < KU; k++) {
-            if (k >= M) break;
-            f[k] = __fdiv_rn(__fsub_rn(obj[(size_t)sol * M + k], ideal[k]), span[k]);
+            for (int k = 0; k < PAD; k += 4)
+                reinterpret_cast<float4 *>(un)[(j * PAD + k) / 4] =
+                    make_float4(w[k] * r, w[k + 1] * r, w[k + 2] * r, w[k + 3] * r);
         }
-        float best = FLT_MAX;
-        int bj = 0;
+    };
+    float f[SOLS][MM], top[SOLS], F[SOLS];
+    int sol[SOLS];
+#pragma unroll
+    for (int q = 0; q < SOLS; q++) {
+        sol[q] = t0 + q < rc ? sc.sorted[t0 + q] : -1;
+        F[q] = 0.0f;
+        top[q] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < MM; k++) {
+            const float ideal = sc.finfo[k], span = __fsub_rn(sc.finfo[2 * MM + k], ideal);
+            f[q][k] = sol[q] >= 0 ? __fdiv_rn(__fsub_rn(obj[(size_t)sol[q] * MM + k], ideal), span) : 0.0f;
+            F[q] = fmaf(f[q][k], f[q][k], F[q]);
+        }
+    }
+    // s^2 of staged point j for solution q
+    auto load = [&](int j, float (&u)[PAD]) {
+#pragma unroll
+        for (int k = 0; k < PAD; k += 4) {
+            const float4 v = reinterpret_cast<const float4 *>(un)[(j * PAD + k) / 4];
+            u[k] = v.x;
+            u[k + 1] = v.y;
+            u[k + 2] = v.z;
+            u[k + 3] = v.w;
+        }
+    };
+    auto square = [&](const float (&u)[PAD], int q) {
+        float x = 0.0f;
+#pragma unroll
+        for (int k = 0; k < MM; k++) x = fmaf(u[k], f[q][k], x);
+        return x * x;
+    };
+    for (int j0 = 0; j0 < R; j0 += chunk) {
+        if (j0) __syncthreads();
+        stage(j0);
+        __syncthreads();
+        const int nc = min(chunk, R - j0);
 #pragma unroll 2
-        for (int j = lane; j < R; j += 32) {
-            const float *w = rp + (size_t)j * M;
-            float num = 0.0f, den = 0.0f;
+        for (int j = lane; j < nc; j += 32) {
+            float u[PAD];
+            load(j, u);
 #pragma unroll
-            for (int k = 0; k < KU; k++) {
-                if (k >= M) break;
-                num = __fadd_rn(num, __fmul_rn(w[k], f[k]));
-                den = __fadd_rn(den, __fmul_rn(w[k], w[k]));
-            }
-            float kk = __fdiv_rn(num, den);
-            float d2 = 0.0f;
-#pragma unroll
-            for (int k = 0; k < KU; k++) {
-                if (k >= M) break;
-                float e = __fsub_rn(__fmul_rn(kk, w[k]), f[k]);
-                d2 = __fadd_rn(d2, __fmul_rn(e, e));
-            }
-            float d = __fsqrt_rn(d2);
-            if (d < best) {
-                best = d;
-                bj = j;
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-            if (ob < best || (ob == best && oj < bj)) {
-                best = ob;
-                bj = oj;
-            }
-        }
-        if (lane == 0) {
-            sc.dist[sol] = best;
-            sc.assoc[t] = bj;
-            atomicAdd(t < count0 ? &sc.rho[bj] : &sc.ncand[bj], 1);
+            for (int q = 0; q < SOLS; q++) top[q] = fmaxf(top[q], square(u, q));
         }
     }
+    float best[SOLS];
+    int bj[SOLS];
+#pragma unroll
+    for (int q = 0; q < SOLS; q++) {
+        // squares are >= +0, so their bits order as they do
+        const float m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top[q])));
+        top[q] = F[q] > 1e-30f && F[q] < 1e30f ? m - kAssocSlack * F[q] : -FLT_MAX;
+        if (sol[q] < 0) top[q] = FLT_MAX;
+        best[q] = FLT_MAX;
+        bj[q] = 0;
+    }
+    for (int j0 = 0; j0 < R; j0 += chunk) {
+        if (chunk < R) {  // one chunk is still in place
+            __syncthreads();
+            stage(j0);
+            __syncthreads();
+        }
+        const int nc = min(chunk, R - j0);
+        for (int j = lane; j < nc; j += 32) {
+            float u[PAD];
+            load(j, u);
+#pragma unroll
+            for (int q = 0; q < SOLS; q++)
+                if (!(square(u, q) < top[q])) {
+                    const float d = assoc_distance<MM>(f[q], refpts + (size_t)(j0 + j) * MM);
+                    if (d < best[q]) {
+                        best[q] = d;
+                        bj[q] = j0 + j;
+                    }
+                }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < SOLS; q++) {
+        // distances are >= +0: the smallest bits, then the lowest index holding them (a
+        // lane that found none holds (FLT_MAX, 0), which the result is when no lane did)
+        const uint32_t b = __float_as_uint(best[q]), mb = __reduce_min_sync(0xffffffffu, b);
+        const uint32_t mj = __reduce_min_sync(0xffffffffu, b == mb ? (uint32_t)bj[q] : 0xffffffffu);
+        if (lane == 0 && sol[q] >= 0) {
+            sc.dist[sol[q]] = __uint_as_float(mb);
+            sc.assoc[t0 + q] = (int)mj;
+            atomicAdd(t0 + q < count0 ? &sc.rho[mj] : &sc.ncand[mj], 1);
+        }
+    }
+}
+
+// A warp takes four solutions (a staged point then serves four) when that still gives
+// every SM a CTA and the points are many, else one: more warps then hide the latency
+// that a short search consists of.
+constexpr int kAssocWideR = 512, kAssocWideN2 = 148 * 8 * 4;
+static bool assoc_wide(const Shape &s) { return s.R >= kAssocWideR && 2 * s.N >= kAssocWideN2; }
+template <int MM, int SOLS>
+static cudaError_t launch_assoc(const Shape &s, const float *obj, const float *refpts, SelectScratch sc, cudaStream_t st)
+{
+    const size_t smem = (size_t)assoc_chunk(s.R, MM) * assoc_pad(MM) * sizeof(float);
+    cudaError_t e = raise_smem_limit((const void *)k_assoc<MM, SOLS>, smem);
+    if (e != cudaSuccess) return e;
+    k_assoc<MM, SOLS><<<(2 * s.N + 8 * SOLS - 1) / (8 * SOLS), 256, smem, st>>>(s, obj, refpts, sc);
+    return cudaGetLastError();
 }
 
 // referenceBasedSorting phase 2 (:1182-1279): candidate lists and niche levels.
@@ -1370,13 +1473,9 @@ cudaError_t launch_select(const Shape &s, const float *obj, float *ext, const fl
         k_select<6><<<1, kSelThreads, smem, st>>>(s, obj, ext, refpts, sc, surv, d_gen, bump_gen);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int warps_needed = 2 * s.N;
-    const int ag = std::min((warps_needed + 7) / 8, 148 * 8);
-    const size_t rb = (size_t)s.R * s.M * sizeof(float), asm_ = rb <= kAssocSmemMax ? rb : 0;
-    if (s.M == 4) k_assoc<4><<<ag, 256, asm_, st>>>(s, obj, refpts, sc);
-    else if (s.M == 6) k_assoc<6><<<ag, 256, asm_, st>>>(s, obj, refpts, sc);
-    else k_assoc<0><<<ag, 256, asm_, st>>>(s, obj, refpts, sc);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (s.M == 4) e = assoc_wide(s) ? launch_assoc<4, 4>(s, obj, refpts, sc, st) : launch_assoc<4, 1>(s, obj, refpts, sc, st);
+    else e = assoc_wide(s) ? launch_assoc<6, 4>(s, obj, refpts, sc, st) : launch_assoc<6, 1>(s, obj, refpts, sc, st);
+    if (e != cudaSuccess) return e;
     const size_t nsm = niche_smem_bytes(s);
     if ((e = raise_smem_limit((const void *)k_niche, nsm)) != cudaSuccess) return e;
     k_niche<<<1, kSelThreads, nsm, st>>>(s, sc, surv, d_gen, bump_gen);
