@@ -1685,7 +1685,15 @@ __device__ void sl_band_scan(const uint4 *__restrict__ E4, const int *__restrict
 // n instead of the n^2/2 cells.  A repetitive CDS makes long chains (many equal
 // words): each thread bounds the nodes and run words it visits, and when any
 // thread passes its bound the CTA drops the partial result and the band scan runs.
-constexpr int kSeedMaxN = 12288;  // longest CDS (nucleotides) with a seeded scan
+// Longest CDS (nucleotides) with a seeded scan: positions and the end mark share 16
+// bits, in the table and in the queue.  The chains grow with n, so the work is
+// n^2 / 12288 chain steps on top of the linear part, against the band scan's n^2 / 2
+// cells: no length at which the band scan would be the better first pass.  The table never
+// decides whether a CDS fits a CTA: the hairpin's (2 n + 16 K bytes) is smaller than the band
+// tables (4.6 n) from n = 6300 on, LRCS's (4 n + 16 K) from n = 27000 on, where
+// both are 124 KB of the 227.  Measured against the former limit of 12288: design
+// runs of 6 x 15003 nucleotides, 100 generations of 1024, 246 -> 94 ms.
+constexpr int kSeedMaxN = 65535;
 constexpr uint32_t kSeedEnd = 0xffffu;
 template <int FL> struct Seed {
     static constexpr int K = FL == 0 ? 6 : 7;  // word length
