@@ -1075,7 +1075,8 @@ __device__ __forceinline__ uint4 shifted_piece(const uint4 *__restrict__ p, int 
 }
 
 // packed: rows x L bytes, 16-byte aligned, readable up to the next multiple of 16;
-// ids: rows x Lp, zero past L.  *bad takes the index of the first id >= 64.
+// ids: rows x Lp, zero past L.  *bad, where given, takes the index of the
+// first id >= 64.
 __global__ void __launch_bounds__(256) k_unpack_rows(const uint8_t *__restrict__ packed, size_t rows, int L, int Lp,
                                                      uint8_t *__restrict__ ids, unsigned long long *bad)
 {
@@ -1093,7 +1094,7 @@ __global__ void __launch_bounds__(256) k_unpack_rows(const uint8_t *__restrict__
             const int k = live - 4 * i;
             if (k < 4) w[i] &= k <= 0 ? 0u : (1u << (8 * k)) - 1u;
         }
-        if ((w[0] | w[1] | w[2] | w[3]) & 0xc0c0c0c0u) {
+        if (bad && ((w[0] | w[1] | w[2] | w[3]) & 0xc0c0c0c0u)) {
             int k = 0;
             while (!((w[k >> 2] >> (8 * (k & 3))) & 0xc0u)) k++;
             atomicMin(bad, (unsigned long long)(at + k));

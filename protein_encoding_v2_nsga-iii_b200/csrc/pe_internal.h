@@ -153,7 +153,7 @@ cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int n
 cudaError_t raise_smem_limit(const void *func, size_t bytes);
 size_t var_smem_bytes(const Shape &s);
 // codon ids from contiguous rows of L bytes (readable up to the next multiple of 16) to
-// rows of Lp, zero past L, *bad (preset to ~0) taking the index of the first id >= 64;
+// rows of Lp, zero past L, *bad (preset to ~0; nullptr: unchecked) taking the index of the first id >= 64;
 // and back.  packed is 16-byte aligned.
 cudaError_t launch_unpack_rows(const uint8_t *packed, size_t rows, int L, int Lp, uint8_t *ids, unsigned long long *bad,
                                cudaStream_t st);

@@ -1,6 +1,7 @@
 """Codon ids on their way between the caller's rows of L bytes and the engine's padded
 rows: row lengths below, at and above multiples of 16, and the refusal of an id out of
-range with the index of the first one."""
+range with the index of the first one, found by the host up to 64 KB of ids (256 x 256
+exactly) and by the device above."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("L,m,n", [(3, 2, 5), (15, 3, 7), (16, 2, 9), (17, 3, 11), (31, 2, 3), (32, 5, 4), (47, 3, 1),
-                                   (257, 2, 21)])
+                                   (257, 2, 21), (256, 2, 128), (257, 2, 128)])
 def test_rows_in_and_out(pe, orc, gpu, L, m, n):
     tabc = pe.dirichlet_table(L)
     tab = tabc.arrays()
