@@ -1679,7 +1679,7 @@ __device__ void sl_band_scan(const uint4 *__restrict__ E4, const int *__restrict
 // heads directly (no hash, no word compare, every node an equal word; 16-bit nodes
 // holding the next position).  LRCS compares CDSs that encode the same protein and
 // share many short words, so it uses K = 7, t = 2 with fewer equal words: hashed
-// 32-bit heads (the power of two >= n, at most 4096) and 32-bit nodes holding the
+// 32-bit heads (sl_seed_heads) and 32-bit nodes holding the
 // word (high half) and the next position (low half).
 //
 // For random-like CDSs the chains hold about n/4096 nodes and the work is linear in
@@ -1702,18 +1702,24 @@ template <int FL> struct Seed {
     static constexpr bool direct = FL == 0;    // the word indexes the heads
 };
 
-__host__ __device__ __forceinline__ int sl_seed_bits(int n, bool direct)
+// heads of the table.  Hashed: the power of two >= n up to 4096, and more for CDSs whose
+// nodes already hold an SM to as many CTAs with them: 6144 from 8193 nucleotides on
+// (three CTAs of 69 KB, as at 4096), 8192 from 12289 on (two), which shortens the chains;
+// past 24576 the nodes need the space.  Design runs of 4 x 9003 nucleotides with
+// N = 4096: 604 -> 560 ms.
+__host__ __device__ __forceinline__ int sl_seed_heads(int n, bool direct)
 {
-    if (direct) return 12;
+    if (direct) return 4096;
+    if (n > 8192 && n <= 24576) return n <= 12288 ? 6144 : 8192;
     int b = 6;
     while ((1 << b) < n && b < 12) b++;
-    return b;
+    return 1 << b;
 }
 __host__ __device__ __forceinline__ bool sl_seeded(const Shape &s) { return s.sl_method == 0 && s.n >= 8 && s.n <= kSeedMaxN; }
 // 32-bit heads, then the nodes (16-bit next positions, or 32-bit word and next)
 __host__ __device__ __forceinline__ size_t sl_seed_head_bytes(int n, bool direct)
 {
-    return ((size_t)1 << sl_seed_bits(n, direct)) * 4;
+    return (size_t)sl_seed_heads(n, direct) * 4;
 }
 __host__ __device__ __forceinline__ size_t sl_seed_bytes(int n, bool direct)
 {
@@ -1729,9 +1735,9 @@ __device__ __forceinline__ uint32_t seed_word(uint32_t lo0, uint32_t lo1, uint32
     if (Seed<FL>::direct) return (fshr(lo0, lo1, sh) & 63u) | ((fshr(hi0, hi1, sh) & 63u) << 6);
     return __byte_perm(fshr(lo0, lo1, sh), fshr(hi0, hi1, sh), 0x4040) & 0x7f7f7f7fu;
 }
-template <int FL> __device__ __forceinline__ uint32_t seed_bucket(uint32_t w, int hb)
+template <int FL> __device__ __forceinline__ uint32_t seed_bucket(uint32_t w, uint32_t heads)
 {
-    return Seed<FL>::direct ? w : (w * 0x9E3779B1u) >> (32 - hb);
+    return Seed<FL>::direct ? w : __umulhi(w * 0x9E3779B1u, heads);
 }
 
 // row p pairs on shift delta (p and p + delta inside [0, n))
@@ -1817,12 +1823,12 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
     constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
     constexpr bool direct = Seed<FL>::direct;
     const int n = geo.n, G = kSlGuardRows, lane = tid & 31;
-    const int hb = sl_seed_bits(n, direct), npos = n - K + 1;  // word starts 0 .. n-K
+    const int nh = sl_seed_heads(n, direct), npos = n - K + 1;  // word starts 0 .. n-K
     uint32_t *heads = reinterpret_cast<uint32_t *>(table);
     unsigned short *next16 = reinterpret_cast<unsigned short *>(table + sl_seed_head_bytes(n, direct));
     uint32_t *node32 = reinterpret_cast<uint32_t *>(table + sl_seed_head_bytes(n, direct));
     uint4 *h4 = reinterpret_cast<uint4 *>(heads);
-    for (int h = tid; h < (1 << hb) / 4; h += nth) h4[h] = make_uint4(kSeedEnd, kSeedEnd, kSeedEnd, kSeedEnd);
+    for (int h = tid; h < nh / 4; h += nth) h4[h] = make_uint4(kSeedEnd, kSeedEnd, kSeedEnd, kSeedEnd);
     __syncthreads();
     // two positions per thread and step, so their exchanges are in flight together
     for (int i = tid; i < npos; i += 2 * nth) {
@@ -1831,8 +1837,8 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
         const int w = (i >> 5) + G, sh = i & 31, w2 = (i2 >> 5) + G, sh2 = i2 & 31;
         const uint32_t c = seed_word<FL>(Tlo[w], Tlo[w + 1], Thi[w], Thi[w + 1], sh);
         const uint32_t c2 = two ? seed_word<FL>(Tlo[w2], Tlo[w2 + 1], Thi[w2], Thi[w2 + 1], sh2) : 0u;
-        const uint32_t old = atomicExch(&heads[seed_bucket<FL>(c, hb)], (uint32_t)i);
-        const uint32_t old2 = two ? atomicExch(&heads[seed_bucket<FL>(c2, hb)], (uint32_t)i2) : 0u;
+        const uint32_t old = atomicExch(&heads[seed_bucket<FL>(c, (uint32_t)nh)], (uint32_t)i);
+        const uint32_t old2 = two ? atomicExch(&heads[seed_bucket<FL>(c2, (uint32_t)nh)], (uint32_t)i2) : 0u;
         if (direct) {
             next16[i] = (unsigned short)old;
             if (two) next16[i2] = (unsigned short)old2;
@@ -1897,13 +1903,13 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
             const int w = a >> 5, sh = a & 31;
             const uint2 s0 = S[w], s1 = S[w + 1];
             c = seed_word<FL>(s0.x, s1.x, s0.y, s1.y, sh);
-            j = heads[seed_bucket<FL>(c, hb)];
+            j = heads[seed_bucket<FL>(c, (uint32_t)nh)];
         }
         if (a2 < npos) {
             const int w = a2 >> 5, sh = a2 & 31;
             const uint2 s0 = S[w], s1 = S[w + 1];
             c2 = seed_word<FL>(s0.x, s1.x, s0.y, s1.y, sh);
-            j2 = heads[seed_bucket<FL>(c2, hb)];
+            j2 = heads[seed_bucket<FL>(c2, (uint32_t)nh)];
         }
         while (__any_sync(0xffffffffu, j != kSeedEnd || j2 != kSeedEnd)) {
             const uint32_t jc = j, jc2 = j2;

@@ -32,3 +32,15 @@ def test_long_stems_match_oracle(pe, orc, gpu):
     ids = rand_ids(np.random.default_rng(L), aa, tabc.arrays(), 2, 1)
     _, handed = check(pe, orc, aa, tabc, ids)
     assert handed == 0
+
+
+@pytest.mark.parametrize("L", [2730, 2731, 4096, 8191, 8192])
+def test_lrcs_head_counts(pe, gpu, L):
+    """CDSs of 3 L nucleotides either side of the lengths where the number of table
+    heads changes (8192, 12288, 24576)."""
+    aa = pe.synthetic_protein(L - 1, L)
+    tab = pe.dirichlet_table(L)
+    pop0, scans0, _ = run(pe, aa, tab, 2, 8, 2, pe.SL_LRCS, 0, 5)
+    pop1, scans1, _ = run(pe, aa, tab, 2, 8, 2, pe.SL_LRCS, 1, 5)
+    assert_same(pop0, pop1)
+    assert scans0 == scans1 > 0
