@@ -1686,15 +1686,21 @@ __device__ void sl_band_scan(const uint4 *__restrict__ E4, const int *__restrict
 // n instead of the n^2/2 cells.  A repetitive CDS makes long chains (many equal
 // words): each thread bounds the nodes and run words it visits, and when any
 // thread passes its bound the CTA drops the partial result and the band scan runs.
+// That bound is some three times the band scan's own time, so CDSs of more than
+// kSeedSampleN nucleotides, where the loss is largest, are sampled first
+// (sl_seed_repetitive).
+//
 // Longest CDS (nucleotides) with a seeded scan: positions and the end mark share 16
-// bits, in the table and in the queue.  The chains grow with n, so the work is
-// n^2 / 12288 chain steps on top of the linear part, against the band scan's n^2 / 2
-// cells: no length at which the band scan would be the better first pass.  The table never
-// decides whether a CDS fits a CTA: the hairpin's (2 n + 16 K bytes) is smaller than the band
-// tables (4.6 n) from n = 6300 on, LRCS's (4 n + 16 K) from n = 27000 on, where
-// both are 124 KB of the 227.  Measured against the former limit of 12288: design
-// runs of 6 x 15003 nucleotides, 100 generations of 1024, 246 -> 94 ms.
+// bits, in the table and in the queue.  The chains of a random-like CDS grow with n, so
+// its work is n / step lookups of n / 4096 nodes (n^2 / 12288 chain steps for the
+// hairpin, n^2 / 8192 for LRCS with 4096 heads) on top of the linear part, against the
+// band scan's n^2 / 2 or n^2 cells.  The table never decides whether a CDS fits a
+// CTA: where it is larger than the band tables (4.6 n bytes; LRCS's 4 n bytes and the
+// heads, up to n = 27000) both are at most 131 KB of the 227.  Measured against
+// the former limit of 12288: design runs of 6 x 15003 nucleotides, 100 generations
+// of 1024, 246 -> 94 ms.
 constexpr int kSeedMaxN = 65535;
+constexpr int kSeedSampleN = 12288;
 constexpr uint32_t kSeedEnd = 0xffffu;
 template <int FL> struct Seed {
     static constexpr int K = FL == 0 ? 6 : 7;  // word length
@@ -1812,13 +1818,53 @@ __device__ __forceinline__ void seed_measure(uint32_t q, const SlGeo &geo, const
     }
 }
 
-// Returns false (CTA-uniform) when some thread passed its bound; (best, bestd) then
-// hold a partial result that the caller discards.  table: the heads, then the nodes;
-// q: this warp's queue, 64 words.
+// Whether a CDS is so repetitive that the band scan is the cheaper pass (CTA-uniform).
+// A warp takes the steps of the longest of its lanes' chains, so what counts is the
+// largest chain of 32 neighbouring lookups: kSeedSamples positions of T, spread by
+// multiples of the golden ratio (no period of the CDS falls in step with them), are counted by
+// bucket in the heads' space, and kSeedBlocks blocks of S's lookups, spread likewise, take
+// the largest count of their 32.  In units of n / kSeedSamples nodes, random-like CDSs
+// have 1.5 - 2.3, CDSs of the best codons alone 2.1 - 4.0, tandem repeats of up to 8 residues
+// 5 - 170; the two passes take the same time at about 4.
+// The sample costs less than 1 % of the band scan; with the bound alone repetitive LRCS
+// designs of 12603 to 27003 nucleotides took 1.8 - 4.4 times the band scan's time, now
+// 0.73 - 1.0.
+// sum: one word of shared memory.
+constexpr int kSeedSamples = 1024, kSeedBlocks = 32, kSeedMostHits = 4;
+template <int FL>
+__device__ bool sl_seed_repetitive(const SlGeo &geo, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
+                                   const uint32_t *__restrict__ Thi, uint32_t *heads, int nh, int *sum, int tid, int nth)
+{
+    constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
+    const int npos = geo.n - K + 1, nlook = (npos + t - 1) / t, lane = tid & 31;
+    uint4 *h4 = reinterpret_cast<uint4 *>(heads);
+    for (int h = tid; h < nh / 4; h += nth) h4[h] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) *sum = 0;
+    __syncthreads();
+    for (int i = tid; i < kSeedSamples; i += nth) {
+        const int p = (int)__umulhi((uint32_t)i * 0x9E3779B1u, (uint32_t)npos), w = (p >> 5) + kSlGuardRows;
+        atomicAdd(&heads[seed_bucket<FL>(seed_word<FL>(Tlo[w], Tlo[w + 1], Thi[w], Thi[w + 1], p & 31), (uint32_t)nh)], 1u);
+    }
+    __syncthreads();
+    uint32_t hits = 0;
+    for (int b = tid >> 5; b < kSeedBlocks; b += nth >> 5) {
+        const int a = t * ((int)__umulhi((uint32_t)b * 0x9E3779B1u, (uint32_t)(nlook - 31)) + lane);  // < npos
+        const uint2 s0 = S[a >> 5], s1 = S[(a >> 5) + 1];
+        hits += __reduce_max_sync(
+            0xffffffffu, heads[seed_bucket<FL>(seed_word<FL>(s0.x, s1.x, s0.y, s1.y, a & 31), (uint32_t)nh)]);
+    }
+    if (lane == 0) atomicAdd(sum, (int)hits);
+    __syncthreads();
+    return *sum > kSeedMostHits * kSeedBlocks;
+}
+
+// Returns false (CTA-uniform) when the CDS is too repetitive or some thread passed its
+// bound; (best, bestd) then hold a partial result that the caller discards.  table:
+// the heads, then the nodes; q: this warp's queue, 64 words; sum: one word of shared memory.
 template <int FL>
 __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
-                             const uint32_t *__restrict__ Thi, unsigned char *table, uint32_t *q, int tid, int nth,
-                             int &best, int &bestd)
+                             const uint32_t *__restrict__ Thi, unsigned char *table, uint32_t *q, int *sum, int tid,
+                             int nth, int &best, int &bestd)
 {
     constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
     constexpr bool direct = Seed<FL>::direct;
@@ -1827,6 +1873,7 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
     uint32_t *heads = reinterpret_cast<uint32_t *>(table);
     unsigned short *next16 = reinterpret_cast<unsigned short *>(table + sl_seed_head_bytes(n, direct));
     uint32_t *node32 = reinterpret_cast<uint32_t *>(table + sl_seed_head_bytes(n, direct));
+    if (n > kSeedSampleN && sl_seed_repetitive<FL>(geo, S, Tlo, Thi, heads, nh, sum, tid, nth)) return false;
     uint4 *h4 = reinterpret_cast<uint4 *>(heads);
     for (int h = tid; h < nh / 4; h += nth) h4[h] = make_uint4(kSeedEnd, kSeedEnd, kSeedEnd, kSeedEnd);
     __syncthreads();
@@ -2104,8 +2151,8 @@ __device__ void sl_item(const Shape &s, PopBuf buf, int base, int2 *part, int32_
         // repetitive CDS) the band scan
         bool band = true;
         if (sl_seeded(s)) {
-            band = !sl_seed_scan<FL>(geo, S, Tlo, Thi, tab, reinterpret_cast<uint32_t *>(sm.queue[warp]), tid, nth, best,
-                                     bestd);
+            band = !sl_seed_scan<FL>(geo, S, Tlo, Thi, tab, reinterpret_cast<uint32_t *>(sm.queue[warp]),
+                                     &sm.next_chunk, tid, nth, best, bestd);
             if (band) {
                 best = 0;
                 bestd = 0x7fffffff;
@@ -2380,8 +2427,10 @@ __global__ void __launch_bounds__(NT) k_sl(Shape s, PopBuf buf, int base, int2 *
 // one wave of CTAs takes them by ticket, the jobs in the order given (longest CDSs
 // first), until all are done.  The last CTA to leave clears the tickets and the
 // counts for the next generation.
+// 256 threads: registers for four CTAs per SM (left alone, the compiler takes 80, three);
+// 0 leaves the smaller sizes to it (64 and 72).
 template <int NT, int FL>
-__global__ void __launch_bounds__(NT) k_sl_queue(const SlJob *__restrict__ jobs, int njobs, int32_t *ticket)
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 0) k_sl_queue(const SlJob *__restrict__ jobs, int njobs, int32_t *ticket)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int qpre[kMaxBatchJobs + 1];
