@@ -80,13 +80,13 @@ L2_FLUSH_BYTES = 256 << 20
 # changes without a new capture.
 SL_NCU = {
     "hairpin": {"workload": "L=1000 m=8 N=1024, generation 1 (2311 CDSs scanned)",
-                "scans": 2311, "cells": 10389102811, "warp_inst": 31038551, "alu_warp_inst": 11606436,
-                "smem_wavefronts": 4299025, "thread_inst": 895579785, "dram_bytes": 2335744,
-                "issue_pct": 64.47, "alu_pct": 46.81, "smem_pct": 29.58, "source": "9732f3c2d57014a7"},
+                "scans": 2311, "cells": 10389102811, "warp_inst": 31266299, "alu_warp_inst": 11443624,
+                "smem_wavefronts": 4297940, "thread_inst": 902906549, "dram_bytes": 2336000,
+                "issue_pct": 65.29, "alu_pct": 46.51, "smem_pct": 28.71, "source": "de797434809ec97a"},
     "lrcs": {"workload": "L=3000 m=4 N=4096, generation 1 (18320 CDS pairs scanned)",
-             "scans": 18320, "cells": 1250515745682, "warp_inst": 1251902908, "alu_warp_inst": 511201202,
-             "smem_wavefronts": 144086701, "thread_inst": 35459069013, "dram_bytes": 31112192,
-             "issue_pct": 45.50, "alu_pct": 37.03, "smem_pct": 20.62, "source": "9732f3c2d57014a7"},
+             "scans": 18320, "cells": 1250515745682, "warp_inst": 1252988385, "alu_warp_inst": 511252021,
+             "smem_wavefronts": 144086714, "thread_inst": 35492477066, "dram_bytes": 31111680,
+             "issue_pct": 44.87, "alu_pct": 36.46, "smem_pct": 20.32, "source": "de797434809ec97a"},
 }
 SM_COUNT, ISSUE_WARP_INST_PER_SM_CLK, SMEM_WAVEFRONTS_PER_SM_CLK, ALU_WARP_INST_PER_SM_CLK = 148, 4, 1, 2
 # kernels one generation launches (one CUDA graph replay): k_variation, k_sl, k_dominance,

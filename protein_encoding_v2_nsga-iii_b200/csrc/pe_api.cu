@@ -560,6 +560,8 @@ int pe_create(const pe_config *cfg, const int8_t *aa_idx, int32_t aa_len, const 
 // and tuned scan CTA size, longest CDSs first
 struct ScanClass {
     int fl = 0, nt = 128, ctas = 0;
+    bool sampled = false;         // some member's CDSs are (sl_sampled)
+    double share = 1.0;           // of the device
     size_t smem = 0;
     std::vector<int> members;
     int32_t *ticket = nullptr;    // [2] device: next item, CTAs done
@@ -599,6 +601,26 @@ static void free_scan_classes(pe_batch *b)
     b->q_count.clear();
 }
 
+// Shared memory and CTAs of a class.
+static cudaError_t size_scan_class(pe_batch *b, ScanClass &k)
+{
+    k.sampled = false;
+    k.smem = 0;
+    for (int i : k.members) {
+        const Shape &s = b->inst[i]->s;
+        k.sampled = k.sampled || sl_sampled(s);
+        k.smem = std::max(k.smem, sl_scan_smem_bytes(s, k.nt, sl_seed_heads(s)));
+    }
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int per_sm = sl_queue_ctas_per_sm(k.nt, k.fl, k.sampled, k.smem);
+    if (per_sm <= 0) return cudaErrorInvalidConfiguration;
+    k.ctas = std::max(1, (int)(k.share * sms * per_sm + 0.5));
+    return cudaSuccess;
+}
+
 // Queues and length classes of the batch's queued scan.  A class is the members with
 // the same string objective and the scan CTA size their init tuning chose; its wave
 // of CTAs is its share of the device, by the members' scan cells per generation.
@@ -626,13 +648,9 @@ static cudaError_t setup_scan_queue(pe_batch *b)
         }
         const int c = cls[key];
         b->classes[c].members.push_back(i);
-        b->classes[c].smem = std::max(b->classes[c].smem, sl_queue_smem_bytes(s, nt));
         work[c] += (double)s.N * s.nres * (double)s.n * s.n;
     }
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     double total = 0.0;
     for (double w : work) total += w;
     for (size_t c = 0; c < b->classes.size(); c++) {
@@ -640,10 +658,8 @@ static cudaError_t setup_scan_queue(pe_batch *b)
         if ((int)k.members.size() > kMaxBatchJobs) return cudaErrorInvalidValue;
         std::sort(k.members.begin(), k.members.end(),
                   [&](int x, int y) { return b->inst[x]->s.n > b->inst[y]->s.n; });
-        const int per_sm = sl_queue_ctas_per_sm(k.nt, k.fl, k.smem);
-        if (per_sm <= 0) return cudaErrorInvalidConfiguration;
-        const double share = total > 0.0 ? work[c] / total : 1.0;
-        k.ctas = std::max(1, (int)(share * sms * per_sm + 0.5));
+        if (total > 0.0) k.share = work[c] / total;
+        if ((e = size_scan_class(b, k)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&k.ticket, 2 * sizeof(int32_t))) != cudaSuccess) return e;
         if ((e = cudaMemset(k.ticket, 0, 2 * sizeof(int32_t))) != cudaSuccess) return e;
         if ((e = cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
@@ -661,6 +677,7 @@ static cudaError_t scan_jobs(pe_batch *b, ScanClass &k, const std::vector<int> &
         pe_instance *in = b->inst[i];
         SlJob &j = h[q];
         j.s = in->s;
+        j.s.sl_heads = sl_seed_heads(j.s);
         j.buf = in->buf[dst[i]];
         j.base = in->s.N;
         j.part = in->d_part;
@@ -741,7 +758,7 @@ static int batch_capture(pe_batch *b, int gens, cudaGraphExec_t *out)
         for (ScanClass &c : b->classes) {
             if (e == cudaSuccess) e = cudaStreamWaitEvent(c.stream, b->fork, 0);
             if (e == cudaSuccess)
-                e = launch_sl_queue(c.jobs[gens][k], (int)c.members.size(), c.ticket, c.nt, c.fl, c.smem, c.ctas,
+                e = launch_sl_queue(c.jobs[gens][k], (int)c.members.size(), c.ticket, c.nt, c.fl, c.sampled, c.smem, c.ctas,
                                     c.stream);
             if (e == cudaSuccess) e = cudaEventRecord(c.done, c.stream);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->master, c.done, 0);

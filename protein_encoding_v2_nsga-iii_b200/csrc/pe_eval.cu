@@ -1679,8 +1679,8 @@ __device__ void sl_band_scan(const uint4 *__restrict__ E4, const int *__restrict
 // heads directly (no hash, no word compare, every node an equal word; 16-bit nodes
 // holding the next position).  LRCS compares CDSs that encode the same protein and
 // share many short words, so it uses K = 7, t = 2 with fewer equal words: hashed
-// 32-bit heads (sl_seed_heads) and 32-bit nodes holding the
-// word (high half) and the next position (low half).
+// 32-bit heads (sl_seed_heads) and 32-bit nodes holding the word (high half) and the
+// next position (low half).
 //
 // For random-like CDSs the chains hold about n/4096 nodes and the work is linear in
 // n instead of the n^2/2 cells.  A repetitive CDS makes long chains (many equal
@@ -1708,28 +1708,13 @@ template <int FL> struct Seed {
     static constexpr bool direct = FL == 0;    // the word indexes the heads
 };
 
-// heads of the table.  Hashed: the power of two >= n up to 4096, and more for CDSs whose
-// nodes already hold an SM to as many CTAs with them: 6144 from 8193 nucleotides on
-// (three CTAs of 69 KB, as at 4096), 8192 from 12289 on (two), which shortens the chains;
-// past 24576 the nodes need the space.  Design runs of 4 x 9003 nucleotides with
-// N = 4096: 604 -> 560 ms.
-__host__ __device__ __forceinline__ int sl_seed_heads(int n, bool direct)
-{
-    if (direct) return 4096;
-    if (n > 8192 && n <= 24576) return n <= 12288 ? 6144 : 8192;
-    int b = 6;
-    while ((1 << b) < n && b < 12) b++;
-    return 1 << b;
-}
 __host__ __device__ __forceinline__ bool sl_seeded(const Shape &s) { return s.sl_method == 0 && s.n >= 8 && s.n <= kSeedMaxN; }
-// 32-bit heads, then the nodes (16-bit next positions, or 32-bit word and next)
-__host__ __device__ __forceinline__ size_t sl_seed_head_bytes(int n, bool direct)
+// 32-bit heads (4096 for the direct table, Shape.sl_heads for the hashed one), then the
+// nodes (16-bit next positions, or 32-bit word and next)
+constexpr int kDirectHeads = 4096;
+__host__ __device__ __forceinline__ size_t sl_seed_bytes(int n, bool direct, int heads)
 {
-    return (size_t)sl_seed_heads(n, direct) * 4;
-}
-__host__ __device__ __forceinline__ size_t sl_seed_bytes(int n, bool direct)
-{
-    return sl_seed_head_bytes(n, direct) + (((size_t)n * (direct ? 2 : 4) + 15) & ~size_t(15));
+    return (size_t)heads * 4 + (((size_t)n * (direct ? 2 : 4) + 15) & ~size_t(15));
 }
 
 // The K-nucleotide word from bit sh of (w0, w1) of both planes: for the direct table
@@ -1821,37 +1806,38 @@ __device__ __forceinline__ void seed_measure(uint32_t q, const SlGeo &geo, const
 // Whether a CDS is so repetitive that the band scan is the cheaper pass (CTA-uniform).
 // A warp takes the steps of the longest of its lanes' chains, so what counts is the
 // largest chain of 32 neighbouring lookups: kSeedSamples positions of T, spread by
-// multiples of the golden ratio (no period of the CDS falls in step with them), are counted by
-// bucket in the heads' space, and kSeedBlocks blocks of S's lookups, spread likewise, take
-// the largest count of their 32.  In units of n / kSeedSamples nodes, random-like CDSs
-// have 1.5 - 2.3, CDSs of the best codons alone 2.1 - 4.0, tandem repeats of up to 8 residues
-// 5 - 170; the two passes take the same time at about 4.
+// multiples of the golden ratio (no period of the CDS falls in step with them), are
+// counted by bucket, and kSeedBlocks blocks of S's lookups, spread likewise, take the largest
+// count of their 32.  In units of n / kSeedSamples nodes, random-like CDSs have 1.5 - 2.3,
+// CDSs of the best codons alone 2.1 - 4.0, tandem repeats of up to 8 residues 5 - 170; the
+// two passes take the same time at about 4.  The counts live in the upper halves of the
+// cleared heads: every bucket that was counted is overwritten when the table is built.
 // The sample costs less than 1 % of the band scan; with the bound alone repetitive LRCS
 // designs of 12603 to 27003 nucleotides took 1.8 - 4.4 times the band scan's time, now
 // 0.73 - 1.0.
-// sum: one word of shared memory.
+// sum: one word of shared memory, cleared.
 constexpr int kSeedSamples = 1024, kSeedBlocks = 32, kSeedMostHits = 4;
-template <int FL>
+template <int NT, int FL>
 __device__ bool sl_seed_repetitive(const SlGeo &geo, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
-                                   const uint32_t *__restrict__ Thi, uint32_t *heads, int nh, int *sum, int tid, int nth)
+                                   const uint32_t *__restrict__ Thi, uint32_t *heads, int nh, int *sum, int tid)
 {
     constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
-    const int npos = geo.n - K + 1, nlook = (npos + t - 1) / t, lane = tid & 31;
-    uint4 *h4 = reinterpret_cast<uint4 *>(heads);
-    for (int h = tid; h < nh / 4; h += nth) h4[h] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) *sum = 0;
-    __syncthreads();
-    for (int i = tid; i < kSeedSamples; i += nth) {
-        const int p = (int)__umulhi((uint32_t)i * 0x9E3779B1u, (uint32_t)npos), w = (p >> 5) + kSlGuardRows;
-        atomicAdd(&heads[seed_bucket<FL>(seed_word<FL>(Tlo[w], Tlo[w + 1], Thi[w], Thi[w + 1], p & 31), (uint32_t)nh)], 1u);
+    const int npos = geo.n - K + 1, nlook = (npos + t - 1) / t, lane = tid & 31, warp = tid >> 5;
+#pragma unroll 4
+    for (int k = 0; k < kSeedSamples / NT; k++) {
+        const int p = (int)__umulhi((uint32_t)(tid + k * NT) * 0x9E3779B1u, (uint32_t)npos), w = (p >> 5) + kSlGuardRows;
+        const uint32_t c = seed_word<FL>(Tlo[w], Tlo[w + 1], Thi[w], Thi[w + 1], p & 31);
+        atomicAdd(&heads[seed_bucket<FL>(c, (uint32_t)nh)], 0x10000u);
     }
     __syncthreads();
     uint32_t hits = 0;
-    for (int b = tid >> 5; b < kSeedBlocks; b += nth >> 5) {
-        const int a = t * ((int)__umulhi((uint32_t)b * 0x9E3779B1u, (uint32_t)(nlook - 31)) + lane);  // < npos
+#pragma unroll 4
+    for (int k = 0; k < 32 * kSeedBlocks / NT; k++) {
+        const uint32_t b = (uint32_t)(warp + k * (NT / 32)) * 0x9E3779B1u;
+        const int a = t * ((int)__umulhi(b, (uint32_t)(nlook - 31)) + lane);  // < npos
         const uint2 s0 = S[a >> 5], s1 = S[(a >> 5) + 1];
-        hits += __reduce_max_sync(
-            0xffffffffu, heads[seed_bucket<FL>(seed_word<FL>(s0.x, s1.x, s0.y, s1.y, a & 31), (uint32_t)nh)]);
+        const uint32_t c = seed_word<FL>(s0.x, s1.x, s0.y, s1.y, a & 31);
+        hits += __reduce_max_sync(0xffffffffu, heads[seed_bucket<FL>(c, (uint32_t)nh)] >> 16);
     }
     if (lane == 0) atomicAdd(sum, (int)hits);
     __syncthreads();
@@ -1860,23 +1846,25 @@ __device__ bool sl_seed_repetitive(const SlGeo &geo, const uint2 *__restrict__ S
 
 // Returns false (CTA-uniform) when the CDS is too repetitive or some thread passed its
 // bound; (best, bestd) then hold a partial result that the caller discards.  table:
-// the heads, then the nodes; q: this warp's queue, 64 words; sum: one word of shared memory.
-template <int FL>
+// nh heads, then the nodes; q: this warp's queue, 64 words; sum: one word of shared memory.
+template <int NT, int FL, bool SAMPLED>
 __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
-                             const uint32_t *__restrict__ Thi, unsigned char *table, uint32_t *q, int *sum, int tid,
-                             int nth, int &best, int &bestd)
+                             const uint32_t *__restrict__ Thi, unsigned char *table, uint32_t *q, int *sum, int nh,
+                             int tid, int nth, int &best, int &bestd)
 {
     constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
     constexpr bool direct = Seed<FL>::direct;
     const int n = geo.n, G = kSlGuardRows, lane = tid & 31;
-    const int nh = sl_seed_heads(n, direct), npos = n - K + 1;  // word starts 0 .. n-K
+    const int npos = n - K + 1;  // word starts 0 .. n-K
     uint32_t *heads = reinterpret_cast<uint32_t *>(table);
-    unsigned short *next16 = reinterpret_cast<unsigned short *>(table + sl_seed_head_bytes(n, direct));
-    uint32_t *node32 = reinterpret_cast<uint32_t *>(table + sl_seed_head_bytes(n, direct));
-    if (n > kSeedSampleN && sl_seed_repetitive<FL>(geo, S, Tlo, Thi, heads, nh, sum, tid, nth)) return false;
+    unsigned short *next16 = reinterpret_cast<unsigned short *>(table + 4 * nh);
+    uint32_t *node32 = reinterpret_cast<uint32_t *>(table + 4 * nh);
     uint4 *h4 = reinterpret_cast<uint4 *>(heads);
     for (int h = tid; h < nh / 4; h += nth) h4[h] = make_uint4(kSeedEnd, kSeedEnd, kSeedEnd, kSeedEnd);
+    const bool sampled = SAMPLED && n > kSeedSampleN;
+    if (sampled && tid == 0) *sum = 0;
     __syncthreads();
+    if (sampled && sl_seed_repetitive<NT, FL>(geo, S, Tlo, Thi, heads, nh, sum, tid)) return false;
     // two positions per thread and step, so their exchanges are in flight together
     for (int i = tid; i < npos; i += 2 * nth) {
         const int i2 = i + nth;
@@ -1890,8 +1878,9 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
             next16[i] = (unsigned short)old;
             if (two) next16[i2] = (unsigned short)old2;
         } else {
-            node32[i] = (c & 0xffff0000u) | old;
-            if (two) node32[i2] = (c2 & 0xffff0000u) | old2;
+            // a head's upper half is 0, or a sample's count
+            node32[i] = (c & 0xffff0000u) | (SAMPLED ? old & 0xffffu : old);
+            if (two) node32[i2] = (c2 & 0xffff0000u) | (SAMPLED ? old2 & 0xffffu : old2);
         }
     }
     __syncthreads();
@@ -2045,7 +2034,9 @@ __device__ __forceinline__ void warp_pick_result(const int2 *res, int count, boo
 // Called by the whole CTA with the CTA's dynamic shared memory.
 // preset: the variation kernel set each child's counter to the results it kept, so a
 // CTA whose result is carried over has nothing to count and leaves at once.
-template <int NT, int FL>
+// SAMPLED: CDSs of more than kSeedSampleN nucleotides are sampled (shorter ones are
+// scanned by kernels without that code, which costs registers).
+template <int NT, int FL, bool SAMPLED>
 __device__ void sl_item(const Shape &s, PopBuf buf, int base, int2 *part, int32_t *counter, int32_t *status,
                         unsigned long long *scanned, int item, unsigned char *smem_raw, bool preset = false)
 {
@@ -2151,8 +2142,8 @@ __device__ void sl_item(const Shape &s, PopBuf buf, int base, int2 *part, int32_
         // repetitive CDS) the band scan
         bool band = true;
         if (sl_seeded(s)) {
-            band = !sl_seed_scan<FL>(geo, S, Tlo, Thi, tab, reinterpret_cast<uint32_t *>(sm.queue[warp]),
-                                     &sm.next_chunk, tid, nth, best, bestd);
+            band = !sl_seed_scan<NT, FL, SAMPLED>(geo, S, Tlo, Thi, tab, reinterpret_cast<uint32_t *>(sm.queue[warp]),
+                                     &sm.next_chunk, FL == 0 ? kDirectHeads : s.sl_heads, tid, nth, best, bestd);
             if (band) {
                 best = 0;
                 bestd = 0x7fffffff;
@@ -2414,12 +2405,12 @@ __device__ void sl_item(const Shape &s, PopBuf buf, int base, int2 *part, int32_
 }
 
 // one CTA per result of solutions base .. base + count - 1
-template <int NT, int FL>
+template <int NT, int FL, bool SAMPLED>
 __global__ void __launch_bounds__(NT) k_sl(Shape s, PopBuf buf, int base, int2 *part, int32_t *counter,
                                                  int32_t *status, unsigned long long *scanned, int preset)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    sl_item<NT, FL>(s, buf, base, part, counter, status, scanned, (int)blockIdx.x, smem_raw, preset != 0);
+    sl_item<NT, FL, SAMPLED>(s, buf, base, part, counter, status, scanned, (int)blockIdx.x, smem_raw, preset != 0);
 }
 
 // The scan items of a whole batch: the variation kernels of the batch's instances
@@ -2427,10 +2418,8 @@ __global__ void __launch_bounds__(NT) k_sl(Shape s, PopBuf buf, int base, int2 *
 // one wave of CTAs takes them by ticket, the jobs in the order given (longest CDSs
 // first), until all are done.  The last CTA to leave clears the tickets and the
 // counts for the next generation.
-// 256 threads: registers for four CTAs per SM (left alone, the compiler takes 80, three);
-// 0 leaves the smaller sizes to it (64 and 72).
-template <int NT, int FL>
-__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 0) k_sl_queue(const SlJob *__restrict__ jobs, int njobs, int32_t *ticket)
+template <int NT, int FL, bool SAMPLED>
+__global__ void __launch_bounds__(NT) k_sl_queue(const SlJob *__restrict__ jobs, int njobs, int32_t *ticket)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int qpre[kMaxBatchJobs + 1];
@@ -2462,7 +2451,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 0) k_sl_queue(const SlJob 
         const int k = cur_job, it = cur_item;
         if (k < 0) break;
         const SlJob &J = jobs[k];
-        sl_item<NT, FL>(J.s, J.buf, J.base, J.part, J.counter, J.status, J.scanned, it, smem_raw);
+        sl_item<NT, FL, SAMPLED>(J.s, J.buf, J.base, J.part, J.counter, J.status, J.scanned, it, smem_raw);
         __syncthreads();  // the next item reuses the shared memory
     }
     if (tid == 0) {
@@ -2577,7 +2566,7 @@ template <int FL> __device__ void lrcs_combine(const Shape &s, PopBuf &buf, size
     }
 }
 
-static size_t sl_smem_bytes_nt(const Shape &s, size_t head)
+static size_t sl_smem_bytes_nt(const Shape &s, size_t head, int heads)
 {
     const int G = kSlGuardRows, W = s.W;
     size_t b = (head + 15) & ~size_t(15);
@@ -2588,72 +2577,91 @@ static size_t sl_smem_bytes_nt(const Shape &s, size_t head)
     const size_t band = (size_t)5 * sl_plane_stride(W) * sizeof(uint4) + (size_t)kSegPitch * (W + 2) * sizeof(int) +
                         (size_t)(ng + 1) * sizeof(int);
     // the two passes share the space
-    b += sl_seeded(s) ? std::max(band, sl_seed_bytes(s.n, s.sl_kind != PE_SL_LRCS)) : band;
+    b += sl_seeded(s) ? std::max(band, sl_seed_bytes(s.n, s.sl_kind != PE_SL_LRCS, heads)) : band;
     return b;
 }
 
-size_t sl_smem_bytes(const Shape &s) { return sl_smem_bytes_nt(s, sizeof(SlSmem<kSlThreadsMax>)); }
-
-// the queued scan's shared memory for a job at CTA size nt
-size_t sl_queue_smem_bytes(const Shape &s, int nt)
+static size_t sl_head_bytes(int nt)
 {
-    switch (nt) {
-    case 64: return sl_smem_bytes_nt(s, sizeof(SlSmem<64>));
-    case 256: return sl_smem_bytes_nt(s, sizeof(SlSmem<256>));
-    default: return sl_smem_bytes_nt(s, sizeof(SlSmem<128>));
-    }
+    return nt == 64 ? sizeof(SlSmem<64>) : nt == 256 ? sizeof(SlSmem<256>) : sizeof(SlSmem<128>);
 }
 
-template <int NT, int FL> static const void *sl_queue_fn() { return (const void *)k_sl_queue<NT, FL>; }
-static const void *sl_queue_kernel(int nt, int fl)
+static int sl_least_heads(const Shape &s)
 {
-    if (fl == 1) return nt == 64 ? sl_queue_fn<64, 1>() : nt == 256 ? sl_queue_fn<256, 1>() : sl_queue_fn<128, 1>();
-    return nt == 64 ? sl_queue_fn<64, 0>() : nt == 256 ? sl_queue_fn<256, 0>() : sl_queue_fn<128, 0>();
+    if (s.sl_kind != PE_SL_LRCS) return kDirectHeads;
+    int heads = 64;
+    while (heads < s.n && heads < 4096) heads *= 2;
+    return heads;
 }
 
-int sl_queue_ctas_per_sm(int nt, int fl, size_t smem)
+size_t sl_scan_smem_bytes(const Shape &s, int nt, int heads) { return sl_smem_bytes_nt(s, sl_head_bytes(nt), heads); }
+
+// Heads of LRCS's hashed table: the power of two >= n up to 4096, 6144 from 8193
+// nucleotides on and 8192 from 12289, which shortens the chains; past 24576 the nodes need
+// the space.  Design runs of 4 x 9003 nucleotides with N = 4096: 604 -> 560 ms.
+int sl_seed_heads(const Shape &s)
 {
-    const void *fn = sl_queue_kernel(nt, fl);
+    if (s.sl_kind == PE_SL_LRCS && s.n > 8192 && s.n <= 24576) return s.n <= 12288 ? 6144 : 8192;
+    return sl_least_heads(s);
+}
+
+size_t sl_smem_bytes(const Shape &s) { return sl_scan_smem_bytes(s, kSlThreadsMax, sl_seed_heads(s)); }
+
+bool sl_sampled(const Shape &s) { return sl_seeded(s) && s.n > kSeedSampleN; }
+
+using QueueKernel = void (*)(const SlJob *, int, int32_t *);
+template <int FL, bool SAMPLED> static QueueKernel sl_queue_of(int nt)
+{
+    return nt == 64 ? k_sl_queue<64, FL, SAMPLED> : nt == 256 ? k_sl_queue<256, FL, SAMPLED> : k_sl_queue<128, FL, SAMPLED>;
+}
+static QueueKernel sl_queue_kernel(int nt, int fl, bool sampled)
+{
+    if (fl == 1) return sampled ? sl_queue_of<1, true>(nt) : sl_queue_of<1, false>(nt);
+    return sampled ? sl_queue_of<0, true>(nt) : sl_queue_of<0, false>(nt);
+}
+
+int sl_queue_ctas_per_sm(int nt, int fl, bool sampled, size_t smem)
+{
+    const void *fn = (const void *)sl_queue_kernel(nt, fl, sampled);
     if (raise_smem_limit(fn, smem) != cudaSuccess) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, nt == 64 || nt == 256 ? nt : 128, smem) != cudaSuccess) return 0;
     return n;
 }
 
-cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int nt, int fl, size_t smem, int ctas,
+cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int nt, int fl, bool sampled, size_t smem, int ctas,
                             cudaStream_t st)
 {
     if (njobs <= 0 || njobs > kMaxBatchJobs || ctas <= 0) return cudaErrorInvalidValue;
-    const void *fn = sl_queue_kernel(nt, fl);
-    cudaError_t e = raise_smem_limit(fn, smem);
+    const QueueKernel fn = sl_queue_kernel(nt, fl, sampled);
+    cudaError_t e = raise_smem_limit((const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    if (fl == 1) {
-        if (nt == 64) k_sl_queue<64, 1><<<ctas, 64, smem, st>>>(jobs, njobs, ticket);
-        else if (nt == 256) k_sl_queue<256, 1><<<ctas, 256, smem, st>>>(jobs, njobs, ticket);
-        else k_sl_queue<128, 1><<<ctas, 128, smem, st>>>(jobs, njobs, ticket);
-    } else {
-        if (nt == 64) k_sl_queue<64, 0><<<ctas, 64, smem, st>>>(jobs, njobs, ticket);
-        else if (nt == 256) k_sl_queue<256, 0><<<ctas, 256, smem, st>>>(jobs, njobs, ticket);
-        else k_sl_queue<128, 0><<<ctas, 128, smem, st>>>(jobs, njobs, ticket);
-    }
+    fn<<<ctas, nt == 64 || nt == 256 ? nt : 128, smem, st>>>(jobs, njobs, ticket);
+    return cudaGetLastError();
+}
+
+template <int NT, int FL, bool SAMPLED>
+static cudaError_t launch_sl_nt(Shape s, PopBuf buf, int base, int count, int2 *part, int32_t *counter, int32_t *status,
+                                cudaStream_t st, unsigned long long *scanned, bool preset)
+{
+    s.sl_heads = sl_seed_heads(s);
+    const size_t smem = sl_scan_smem_bytes(s, NT, s.sl_heads);
+    cudaError_t e = raise_smem_limit((const void *)k_sl<NT, FL, SAMPLED>, smem);
+    if (e != cudaSuccess) return e;
+    k_sl<NT, FL, SAMPLED><<<count * (FL == 0 ? s.m : s.nres), NT, smem, st>>>(s, buf, base, part, counter, status, scanned,
+                                                                              (int)preset);
     return cudaGetLastError();
 }
 
 template <int NT>
-static cudaError_t launch_sl_nt(const Shape &s, PopBuf buf, int base, int count, int2 *part, int32_t *counter,
+static cudaError_t launch_sl_of(const Shape &s, PopBuf buf, int base, int count, int2 *part, int32_t *counter,
                                 int32_t *status, cudaStream_t st, unsigned long long *scanned, bool preset)
 {
-    const size_t smem = sl_smem_bytes_nt(s, sizeof(SlSmem<NT>));
-    if (s.sl_kind == PE_SL_LRCS) {
-        cudaError_t e = raise_smem_limit((const void *)k_sl<NT, 1>, smem);
-        if (e != cudaSuccess) return e;
-        k_sl<NT, 1><<<count * s.nres, NT, smem, st>>>(s, buf, base, part, counter, status, scanned, (int)preset);
-        return cudaGetLastError();
-    }
-    cudaError_t e = raise_smem_limit((const void *)k_sl<NT, 0>, smem);
-    if (e != cudaSuccess) return e;
-    k_sl<NT, 0><<<count * s.m, NT, smem, st>>>(s, buf, base, part, counter, status, scanned, (int)preset);
-    return cudaGetLastError();
+    if (s.sl_kind == PE_SL_LRCS)
+        return (sl_sampled(s) ? launch_sl_nt<NT, 1, true> : launch_sl_nt<NT, 1, false>)(s, buf, base, count, part, counter,
+                                                                                     status, st, scanned, preset);
+    return (sl_sampled(s) ? launch_sl_nt<NT, 0, true> : launch_sl_nt<NT, 0, false>)(s, buf, base, count, part, counter,
+                                                                                 status, st, scanned, preset);
 }
 
 cudaError_t launch_sl(const Shape &s, PopBuf buf, int base, int count, int2 *part, int32_t *counter, int32_t *status,
@@ -2661,9 +2669,9 @@ cudaError_t launch_sl(const Shape &s, PopBuf buf, int base, int count, int2 *par
 {
     if (count <= 0) return cudaSuccess;
     switch (s.sl_threads) {
-    case 64: return launch_sl_nt<64>(s, buf, base, count, part, counter, status, st, scanned, preset);
-    case 256: return launch_sl_nt<256>(s, buf, base, count, part, counter, status, st, scanned, preset);
-    default: return launch_sl_nt<128>(s, buf, base, count, part, counter, status, st, scanned, preset);
+    case 64: return launch_sl_of<64>(s, buf, base, count, part, counter, status, st, scanned, preset);
+    case 256: return launch_sl_of<256>(s, buf, base, count, part, counter, status, st, scanned, preset);
+    default: return launch_sl_of<128>(s, buf, base, count, part, counter, status, st, scanned, preset);
     }
 }
 

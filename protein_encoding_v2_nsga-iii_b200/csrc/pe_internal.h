@@ -43,6 +43,7 @@ struct Shape {
     int wait_limit;  // polls of a bounded device wait: 0 = the default, < 0 = give up at once (tests)
     int naux;        // int32 words of per-CDS sums per solution: AUX_HD(m) + m(m-1)/2
     int sl_method;   // first pass of the string scan: 0 seeded (word table) where the CDS fits, 1 band scan
+    int sl_heads;    // heads of the LRCS scan's table, set for each launch (sl_seed_heads)
 };
 
 // Per-solution sums of the light objectives (PopBuf.aux), int32 words: per CDS c the
@@ -141,11 +142,16 @@ cudaError_t launch_mutate(const Shape &s, const DevTables *tab, const int8_t *aa
 cudaError_t launch_sl(const Shape &s, PopBuf buf, int base, int count, int2 *part, int32_t *counter,
                       int32_t *status, cudaStream_t st, unsigned long long *scanned = nullptr, bool preset = false);
 size_t sl_smem_bytes(const Shape &s);
-// the batch's queued stem scan (k_sl_queue): shared memory of a job at CTA size nt,
-// resident CTAs per SM, and the launch of one wave over jobs[0 .. njobs)
-size_t sl_queue_smem_bytes(const Shape &s, int nt);
-int sl_queue_ctas_per_sm(int nt, int fl, size_t smem);
-cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int nt, int fl, size_t smem, int ctas,
+// dynamic shared memory of a scan CTA of nt threads whose table has `heads` heads, and the
+// heads it has (for the queue the caller puts them into SlJob.s)
+int sl_seed_heads(const Shape &s);
+size_t sl_scan_smem_bytes(const Shape &s, int nt, int heads);
+// whether the shape's CDSs are long enough to be sampled before the seeded scan
+bool sl_sampled(const Shape &s);
+// the batch's queued stem scan (k_sl_queue): resident CTAs per SM, and the launch of one
+// wave over jobs[0 .. njobs); sampled: some job's CDSs are (sl_sampled)
+int sl_queue_ctas_per_sm(int nt, int fl, bool sampled, size_t smem);
+cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int nt, int fl, bool sampled, size_t smem, int ctas,
                             cudaStream_t st);
 // Raise a kernel's dynamic shared-memory limit to at least `bytes` on the current
 // device.  The limit only grows, so launches from different host threads never
