@@ -560,6 +560,7 @@ int pe_create(const pe_config *cfg, const int8_t *aa_idx, int32_t aa_len, const 
 // and tuned scan CTA size, longest CDSs first
 struct ScanClass {
     int fl = 0, nt = 128, ctas = 0;
+    int per_sm = 0;               // CTAs per SM that the members' smallest tables allow
     bool sampled = false;         // some member's CDSs are (sl_sampled)
     double share = 1.0;           // of the device
     size_t smem = 0;
@@ -601,15 +602,22 @@ static void free_scan_classes(pe_batch *b)
     b->q_count.clear();
 }
 
-// Shared memory and CTAs of a class.
+// Shared memory, table heads and CTAs of a class.  Its members share a launch, so the
+// largest member decides how many CTAs an SM holds, and every member's table takes what
+// that leaves.
 static cudaError_t size_scan_class(pe_batch *b, ScanClass &k)
 {
+    k.per_sm = 1 << 30;
     k.sampled = false;
     k.smem = 0;
     for (int i : k.members) {
         const Shape &s = b->inst[i]->s;
+        k.per_sm = std::min(k.per_sm, sl_scan_ctas(s, k.nt, true));
         k.sampled = k.sampled || sl_sampled(s);
-        k.smem = std::max(k.smem, sl_scan_smem_bytes(s, k.nt, sl_seed_heads(s)));
+    }
+    for (int i : k.members) {
+        const Shape &s = b->inst[i]->s;
+        k.smem = std::max(k.smem, sl_scan_smem_bytes(s, k.nt, sl_seed_heads(s, k.nt, true, k.per_sm)));
     }
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -677,7 +685,7 @@ static cudaError_t scan_jobs(pe_batch *b, ScanClass &k, const std::vector<int> &
         pe_instance *in = b->inst[i];
         SlJob &j = h[q];
         j.s = in->s;
-        j.s.sl_heads = sl_seed_heads(j.s);
+        j.s.sl_heads = sl_seed_heads(j.s, k.nt, true, k.per_sm);
         j.buf = in->buf[dst[i]];
         j.base = in->s.N;
         j.part = in->d_part;

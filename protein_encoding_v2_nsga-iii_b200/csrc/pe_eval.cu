@@ -2586,6 +2586,14 @@ static size_t sl_head_bytes(int nt)
     return nt == 64 ? sizeof(SlSmem<64>) : nt == 256 ? sizeof(SlSmem<256>) : sizeof(SlSmem<128>);
 }
 
+// CTAs per SM by shared memory alone (228 KB, of which a CTA also takes 1 KB for the
+// system), for a CTA of `bytes` dynamic and `fixed` static bytes
+static int sl_ctas_by_smem(size_t bytes, size_t fixed)
+{
+    return (int)(228 * 1024 / (((bytes + fixed + 127) & ~size_t(127)) + 1024));
+}
+constexpr size_t kScanStatic = 16, kQueueStatic = 4128;  // static shared bytes of k_sl, k_sl_queue
+
 static int sl_least_heads(const Shape &s)
 {
     if (s.sl_kind != PE_SL_LRCS) return kDirectHeads;
@@ -2596,16 +2604,31 @@ static int sl_least_heads(const Shape &s)
 
 size_t sl_scan_smem_bytes(const Shape &s, int nt, int heads) { return sl_smem_bytes_nt(s, sl_head_bytes(nt), heads); }
 
-// Heads of LRCS's hashed table: the power of two >= n up to 4096, 6144 from 8193
-// nucleotides on and 8192 from 12289, which shortens the chains; past 24576 the nodes need
-// the space.  Design runs of 4 x 9003 nucleotides with N = 4096: 604 -> 560 ms.
-int sl_seed_heads(const Shape &s)
+int sl_scan_ctas(const Shape &s, int nt, bool queue)
 {
-    if (s.sl_kind == PE_SL_LRCS && s.n > 8192 && s.n <= 24576) return s.n <= 12288 ? 6144 : 8192;
-    return sl_least_heads(s);
+    return sl_ctas_by_smem(sl_scan_smem_bytes(s, nt, sl_least_heads(s)), queue ? kQueueStatic : kScanStatic);
 }
 
-size_t sl_smem_bytes(const Shape &s) { return sl_scan_smem_bytes(s, kSlThreadsMax, sl_seed_heads(s)); }
+// Heads of LRCS's hashed table: the power of two >= n up to 4096, and above 8192
+// nucleotides the most of 4096, 6144 and 8192 that leave an SM `ctas` CTAs.  The callers
+// ask for what 4096 leave, or for fewer where the launch has no more: the scan is a
+// chain of dependent shared-memory loads, so more heads (shorter chains) pay only while no
+// CTA is lost for them.  Generations of 512 designs of two CDSs, 256 threads, with
+// 4096 heads and with this rule's: 9003 nucleotides 0.221 -> 0.207 ms (6144, three CTAs both
+// ways), 13803 0.427 -> 0.385 (8192, two), 24903 1.40 -> 1.18 (8192, one).  At 11703, 6144
+// heads (two CTAs instead of three) take 0.311 against 0.298, at 18603, 8192 (one instead of
+// two) 0.780 against 0.620; with 128 designs, which fill one CTA per SM, 12273 nucleotides
+// take 0.204 with 4096 heads and 0.178 with 6144.
+int sl_seed_heads(const Shape &s, int nt, bool queue, int ctas)
+{
+    const int heads = sl_least_heads(s);
+    if (s.sl_kind == PE_SL_LRCS && s.n > 8192)
+        for (int more = 8192; more > heads; more -= 2048)
+            if (sl_ctas_by_smem(sl_scan_smem_bytes(s, nt, more), queue ? kQueueStatic : kScanStatic) >= ctas) return more;
+    return heads;
+}
+
+size_t sl_smem_bytes(const Shape &s) { return sl_scan_smem_bytes(s, kSlThreadsMax, sl_least_heads(s)); }
 
 bool sl_sampled(const Shape &s) { return sl_seeded(s) && s.n > kSeedSampleN; }
 
@@ -2644,7 +2667,11 @@ template <int NT, int FL, bool SAMPLED>
 static cudaError_t launch_sl_nt(Shape s, PopBuf buf, int base, int count, int2 *part, int32_t *counter, int32_t *status,
                                 cudaStream_t st, unsigned long long *scanned, bool preset)
 {
-    s.sl_heads = sl_seed_heads(s);
+    // CTAs per SM that the launch can use: a generation's scans are half of its results or
+    // fewer (the others are carried over)
+    const int64_t scans = ((int64_t)count * (FL == 0 ? s.m : s.nres) + preset) / (1 + preset);
+    const int use = (int)std::min<int64_t>(sl_scan_ctas(s, NT, false), (scans + 147) / 148);
+    s.sl_heads = sl_seed_heads(s, NT, false, use);
     const size_t smem = sl_scan_smem_bytes(s, NT, s.sl_heads);
     cudaError_t e = raise_smem_limit((const void *)k_sl<NT, FL, SAMPLED>, smem);
     if (e != cudaSuccess) return e;

@@ -142,9 +142,12 @@ cudaError_t launch_mutate(const Shape &s, const DevTables *tab, const int8_t *aa
 cudaError_t launch_sl(const Shape &s, PopBuf buf, int base, int count, int2 *part, int32_t *counter,
                       int32_t *status, cudaStream_t st, unsigned long long *scanned = nullptr, bool preset = false);
 size_t sl_smem_bytes(const Shape &s);
-// dynamic shared memory of a scan CTA of nt threads whose table has `heads` heads, and the
-// heads it has (for the queue the caller puts them into SlJob.s)
-int sl_seed_heads(const Shape &s);
+// A scan CTA of nt threads (of k_sl, or of k_sl_queue): how often it fits an SM by its
+// shared memory with the smallest table, the heads of the largest table with which it still
+// fits `ctas` times (for the queue the caller puts them into SlJob.s), and its dynamic
+// shared memory with them.
+int sl_scan_ctas(const Shape &s, int nt, bool queue);
+int sl_seed_heads(const Shape &s, int nt, bool queue, int ctas);
 size_t sl_scan_smem_bytes(const Shape &s, int nt, int heads);
 // whether the shape's CDSs are long enough to be sampled before the seeded scan
 bool sl_sampled(const Shape &s);
