@@ -667,7 +667,6 @@ static cudaError_t setup_scan_queue(pe_batch *b)
         std::sort(k.members.begin(), k.members.end(),
                   [&](int x, int y) { return b->inst[x]->s.n > b->inst[y]->s.n; });
         if (total > 0.0) k.share = work[c] / total;
-        if ((e = size_scan_class(b, k)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&k.ticket, 2 * sizeof(int32_t))) != cudaSuccess) return e;
         if ((e = cudaMemset(k.ticket, 0, 2 * sizeof(int32_t))) != cudaSuccess) return e;
         if ((e = cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
@@ -728,6 +727,10 @@ static int batch_capture(pe_batch *b, int gens, cudaGraphExec_t *out)
             return fail(PE_ERR_CUDA, "batch scan queue setup: %s", cudaGetErrorString(e0));
         }
     }
+    // The members' shapes may have changed since the last capture (pe_set_scan_method), and
+    // with them the shared memory that their scans take; a captured graph keeps its own.
+    if (b->queue)
+        for (ScanClass &c : b->classes) CK(size_scan_class(b, c));
     if (b->queue) {  // the job tables of each step, before the capture
         std::vector<int> s2 = src;
         for (int k = 0; k < gens; k++) {
