@@ -732,6 +732,8 @@ static int batch_capture(pe_batch *b, int gens, cudaGraphExec_t *out)
     if (b->queue)
         for (ScanClass &c : b->classes) CK(size_scan_class(b, c));
     if (b->queue) {  // the job tables of each step, before the capture
+        // an earlier graph of this step count may still be reading them
+        CK(cudaStreamSynchronize(b->master));
         std::vector<int> s2 = src;
         for (int k = 0; k < gens; k++) {
             std::vector<int> dst(n);

@@ -1,5 +1,6 @@
 """A batch's queued scan when its graphs are captured again: with members whose scan
-method changed since the first capture (other tables, other shared memory)."""
+method changed since the first capture (other tables, other shared memory), and while
+the generations of the graph that it replaces are still running."""
 import pytest
 
 from test_gpu_batch import population_equal
@@ -45,6 +46,26 @@ def test_scan_method_changed_between_captures(pe, gpu, first):
             e.set_scan_method(1 - first)
         b.step(1)
         b.step(2)
+        b.synchronize()
+    for e, w in zip(engines, want):
+        assert population_equal(e.population(), w)
+        e.close()
+
+
+def test_captured_again_while_running(pe, gpu):
+    """Steps of 2 + 1 and 2 generations, queued without waiting: the second capture of the
+    two-generation graph (the buffers' parity changed) writes job tables that the first
+    one's generations, some milliseconds each, may not have read yet."""
+    jobs = [(6000, 4, 512, 64, pe.SL_LRCS), (300, 2, 64, 64, pe.SL_LRCS)]
+    want = alone(pe, jobs, 8)
+    engines = engines_of(pe, jobs)
+    for e in engines:
+        e.init()
+    with pe.Batch(engines) as b:
+        b.set_scan_queue(True)
+        b.step(3)
+        b.step(2)
+        b.step(3)
         b.synchronize()
     for e, w in zip(engines, want):
         assert population_equal(e.population(), w)
