@@ -506,10 +506,10 @@ int pe_create(const pe_config *cfg, const int8_t *aa_idx, int32_t aa_len, const 
     if ((rc = in->alloc(&in->d_ref, (size_t)s.R * s.M))) return cleanup(rc);
     for (int b = 0; b < 2; b++)
         if ((rc = alloc_pop(in, in->buf[b], 2 * N))) return cleanup(rc);
-    const int N2 = 2 * N, words = (N2 + 31) / 32;
+    const int N2 = 2 * N;
     if ((rc = in->alloc(&in->d_surv, (size_t)N))) return cleanup(rc);
     if ((rc = in->alloc(&in->d_order, (size_t)2 * N))) return cleanup(rc);
-    if ((rc = in->alloc(&in->sc.dom, (size_t)N2 * words))) return cleanup(rc);
+    if ((rc = in->alloc(&in->sc.dom, dom_matrix_words(N2)))) return cleanup(rc);
     if ((rc = in->alloc(&in->sc.np, (size_t)N2 * dom_tile_count(N2)))) return cleanup(rc);
     if ((rc = in->alloc(&in->sc.front, (size_t)N2))) return cleanup(rc);
     if ((rc = in->alloc(&in->sc.sorted, (size_t)N2))) return cleanup(rc);
@@ -1002,11 +1002,11 @@ int pe_instance_bytes(const pe_config *cfg, int32_t aa_len, uint64_t *bytes)
         p -= 1;
         if (p < 1) return fail(PE_ERR_ARG, "pop_size too small for the reference-point rule");
     }
-    const uint64_t R = bincoef((int)M + p - 1, p), words = (N2 + 31) / 32;
+    const uint64_t R = bincoef((int)M + p - 1, p);
     auto r = [](uint64_t b) { return (b + 511) & ~uint64_t(511); };  // allocation granularity
     uint64_t t = r(sizeof(DevTables)) + r(L) + r(R * M * 4);
     t += 2 * (r(N2 * m * Lp) + r(N2 * m * Wp * 8) + r(N2 * M * 4) + r(N2 * 2 * M) + r(N2 * 12));
-    t += r(N * 4) + r(N2 * 4) + r(N2 * words * 4) + r(N2 * (uint64_t)dom_tile_count((int)N2) * 4) + 4 * r(N2 * 4) +
+    t += r(N * 4) + r(N2 * 4) + r((uint64_t)dom_matrix_words((int)N2) * 4) + r(N2 * (uint64_t)dom_tile_count((int)N2) * 4) + 4 * r(N2 * 4) +
          2 * r(R * 4) + r((N2 + M) * 4) + r(32) + r(72);
     const uint64_t nres = cfg->sl_kind == PE_SL_LRCS ? m * (m + 1) / 2 : m;
     t += r(N2 * nres * 8) + r(N2 * 4) + r(4) + r(M * M * 4) + r(4);

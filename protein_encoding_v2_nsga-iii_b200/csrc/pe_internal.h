@@ -99,7 +99,7 @@ struct PopBuf {
 };
 
 struct SelectScratch {
-    uint32_t *dom;       // [2N][2N/32] bit j of row i: j dominates i
+    uint32_t *dom;       // [2N][2N/32, rounded up to 4] bit j of row i: j dominates i
     int32_t *np;         // [column tiles][2N] dominators of each row per tile of the matrix
     int32_t *front;      // [2N]
     int32_t *sorted;     // [2N] fronts 0..last
@@ -108,7 +108,7 @@ struct SelectScratch {
     int32_t *rho;        // [R]
     int32_t *ncand;      // [R]
     uint32_t *trank;     // [2N + M] place of each extreme-point search position in the reduction-tree order
-    int32_t *info;       // [8] rank_count, last_size, n_fronts, cut, hyp_exc, status
+    int32_t *info;       // [8] rank_count, last_size, n_fronts, cut, hyp_exc, first place of the last front
     float *finfo;        // [3*M] ideal, worst, nadir
 };
 
@@ -177,6 +177,8 @@ cudaError_t launch_select(const Shape &s, const float *obj, float *ext, const fl
 size_t select_smem_bytes(const Shape &s);
 // column tiles of the dominance matrix: SelectScratch.np holds 2N x this many counts
 int dom_tile_count(int N2);
+// words of the dominance matrix
+size_t dom_matrix_words(int N2);
 size_t niche_smem_bytes(const Shape &s);
 // place of every position 0 .. B-1 of the extreme-point search in the reference's
 // reduction-tree order (0xffffffff: a position the tree leaves out)

@@ -61,13 +61,15 @@ __device__ __forceinline__ bool dominates(const float (&a)[MM], const float (&b)
 // (6.7 us at 2048 solutions, 52.7 at 8192, of
 // four objectives; 8.0 and 59.5 before).  MM: the objective count (4 or 6).
 constexpr int kDomTileWords = 8;
+// words of a row of the matrix: whole 16-byte pieces for the peeling
+__host__ __device__ inline int dom_stride(int N2) { return (((N2 + 31) >> 5) + 3) & ~3; }
 template <int MM>
 __global__ void __launch_bounds__(32 * kDomTileWords) k_dominance(Shape s, const float *__restrict__ obj,
                                                                   uint32_t *__restrict__ dom, int32_t *__restrict__ np)
 {
     __shared__ __align__(16) float oc[32 * kDomTileWords * MM];  // tile columns, objective vectors in column order
     __shared__ uint32_t tw[32][kDomTileWords + 1];               // the tile's words by row
-    const int N2 = 2 * s.N, words = (N2 + 31) >> 5;
+    const int N2 = 2 * s.N, words = (N2 + 31) >> 5, stride = dom_stride(N2);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i = blockIdx.x * 32 + lane, j0 = blockIdx.y * 32 * kDomTileWords;
     const int ncol = min(32 * kDomTileWords, N2 - j0);
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(32 * kDomTileWords) k_dominance(Shape s, const
     {
         const int r = tid / kDomTileWords, w = tid % kDomTileWords;
         const int row = blockIdx.x * 32 + r, wd2 = blockIdx.y * kDomTileWords + w;
-        if (row < N2 && wd2 < words) dom[(size_t)row * words + wd2] = tw[r][w];
+        if (row < N2 && wd2 < stride) dom[(size_t)row * stride + wd2] = tw[r][w];  // 0 past the last word
     }
     if (tid < 32) {
         int cnt = 0;
@@ -521,11 +523,11 @@ __device__ __forceinline__ void peel_fronts(const Shape &s, const SelectScratch 
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ int s_warp[32];
     const int c = (int)cluster.block_rank();
-    const int N = s.N, N2 = 2 * N, words = (N2 + 31) >> 5;
+    const int N = s.N, N2 = 2 * N, words = (N2 + 31) >> 5, stride = dom_stride(N2);
     const int RR = front_rows_per_cta(N2), sw = RR >> 5;
     const int r0 = c * RR, nrow = max(0, min(N2, r0 + RR) - r0);
-    uint32_t *fmask = reinterpret_cast<uint32_t *>(fsm_raw);          // words: the current front
-    uint32_t *slice = fmask + ((words + 3) & ~3);                      // [2][sw]: own rows joining a front
+    uint32_t *fmask = reinterpret_cast<uint32_t *>(fsm_raw);          // stride: the current front, 0 past its words
+    uint32_t *slice = fmask + stride;                                  // [2][sw]: own rows joining a front
     int *npr = reinterpret_cast<int *>(slice + 2 * ((sw + 3) & ~3));   // [RR]: unassigned dominators
     int *wpre = npr + RR;                                              // [words]: members before each word
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nth >> 5;
@@ -543,6 +545,7 @@ __device__ __forceinline__ void peel_fronts(const Shape &s, const SelectScratch 
         if (q < nrow) sc.front[r0 + q] = -1;
     }
     for (int w = tid; w < 2 * swp; w += nth) slice[w] = 0u;
+    for (int w = words + tid; w < stride; w += nth) fmask[w] = 0u;
     __syncthreads();
     for (int q = tid; q < nrow; q += nth)
         if (npr[q] == 0) atomicOr(&slice[q >> 5], 1u << (q & 31));
@@ -606,8 +609,8 @@ __device__ __forceinline__ void peel_fronts(const Shape &s, const SelectScratch 
         __syncthreads();
         // eight rows per warp at a time, so their loads are in flight together
         for (int q0 = warp; q0 < nrow; q0 += 8 * nwarps) {
-            const uint32_t *base = sc.dom + (size_t)(r0 + q0) * words;
-            const size_t step = (size_t)nwarps * words;  // between the warp's rows u and u+1
+            const uint4 *base = reinterpret_cast<const uint4 *>(sc.dom + (size_t)(r0 + q0) * stride);
+            const size_t step = (size_t)nwarps * (stride >> 2);  // between the warp's rows u and u+1
             unsigned act = 0u;
             int dec[8];
 #pragma unroll
@@ -617,27 +620,17 @@ __device__ __forceinline__ void peel_fronts(const Shape &s, const SelectScratch 
                 dec[u] = 0;
             }
             if (!act) continue;
-            if ((words & 3) == 0) {  // whole 16-byte pieces: four times the bytes in flight (selection of 8192
-                                     // solutions 512 -> 393 us)
-                const uint4 *base4 = reinterpret_cast<const uint4 *>(base);
-                for (int w = lane; w < (words >> 2); w += 32) {
-                    const uint4 f = reinterpret_cast<const uint4 *>(fmask)[w];
-                    if (!(f.x | f.y | f.z | f.w)) continue;
+            // 16-byte pieces, four times the bytes in flight of single words (selection of 8192
+            // solutions 512 -> 393 us; of 8000, whose rows are 250 words, 458 -> 367)
+            for (int w = lane; w < (stride >> 2); w += 32) {
+                const uint4 f = reinterpret_cast<const uint4 *>(fmask)[w];
+                if (!(f.x | f.y | f.z | f.w)) continue;
 #pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (act & (1u << u)) {
-                            const uint4 v = __ldg(base4 + u * (step >> 2) + w);
-                            dec[u] += __popc(v.x & f.x) + __popc(v.y & f.y) + __popc(v.z & f.z) + __popc(v.w & f.w);
-                        }
-                }
-            } else {
-                for (int w = lane; w < words; w += 32) {
-                    const uint32_t f = fmask[w];
-                    if (!f) continue;
-#pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (act & (1u << u)) dec[u] += __popc(__ldg(base + u * step + w) & f);
-                }
+                for (int u = 0; u < 8; u++)
+                    if (act & (1u << u)) {
+                        const uint4 v = __ldg(base + u * step + w);
+                        dec[u] += __popc(v.x & f.x) + __popc(v.y & f.y) + __popc(v.z & f.z) + __popc(v.w & f.w);
+                    }
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
@@ -667,7 +660,7 @@ __device__ __forceinline__ void peel_fronts(const Shape &s, const SelectScratch 
 size_t fronts_smem_bytes(const Shape &s)
 {
     const int N2 = 2 * s.N, words = (N2 + 31) >> 5, RR = front_rows_per_cta(N2), sw = RR >> 5;
-    return (size_t)((words + 3) & ~3) * 4 + (size_t)2 * ((sw + 3) & ~3) * 4 + (size_t)RR * 4 + (size_t)words * 4;
+    return (size_t)dom_stride(N2) * 4 + (size_t)2 * ((sw + 3) & ~3) * 4 + (size_t)RR * 4 + (size_t)words * 4;
 }
 
 // Ideal, worst and extreme points and the hyperplane's (or the fallback's) nadir by one
@@ -1479,6 +1472,7 @@ size_t niche_smem_bytes(const Shape &s)
 }
 
 int dom_tile_count(int N2) { return dom_tiles(N2); }
+size_t dom_matrix_words(int N2) { return (size_t)N2 * dom_stride(N2); }
 
 size_t select_smem_bytes(const Shape &s)
 {
