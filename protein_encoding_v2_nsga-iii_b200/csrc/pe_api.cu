@@ -7,7 +7,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -217,10 +219,18 @@ int alloc_pop(pe_instance *in, PopBuf &b, int nsol)
 struct TempBufs {
     const pe_instance *in;
     std::vector<void *> v;
+    std::vector<std::unique_ptr<uint8_t[]>> h;
     explicit TempBufs(const pe_instance *in_) : in(in_) {}
     ~TempBufs()
     {
         for (void *p : v) cudaFreeAsync(p, in->stream);
+    }
+    // host memory that lives as long as the device buffers
+    int host(uint8_t **p, size_t bytes)
+    {
+        h.emplace_back(new (std::nothrow) uint8_t[bytes]);
+        *p = h.back().get();
+        return *p ? PE_OK : fail(PE_ERR_OOM, "host allocation of %zu bytes", bytes);
     }
     template <class T> int get(T **p, size_t count)
     {
@@ -1197,19 +1207,23 @@ int pe_read_objectives_async(pe_instance *in, float *obj)
     return PE_OK;
 }
 
-// The caller's n x m rows of L codon ids into device rows of Lp by way of `staging` (n m L
-// bytes, rounded up to 16), checked there: an id out of range ends the call before
-// anything else ran on it.  With a checking loop on the host and a pitched copy in its
-// place, scoring 1024 solutions of 8 x 1001 codons took 7.1 - 10.8 ms a call; now 1.1 ms.
-// Up to kHostCheckBytes the host checks them, eight at a time: the device's answer costs a
-// copy back and a wait, about 11 us, which is what the host's pass over 64 KB costs at most.
-constexpr size_t kHostCheckBytes = 64 * 1024;
-static int upload_ids(pe_instance *in, const uint8_t *host, size_t rows, uint8_t *staging, uint8_t *ids,
-                      unsigned long long *d_bad)
+// The caller's rows of L codon ids into device rows of Lp, checked: an id out of range ends
+// the call before anything else ran on it.
+//
+// Up to kHostRowBytes (of Lp bytes a row) the host checks the ids, eight at a time, and pads
+// the rows itself, so the device gets one copy: 51 codons x 2 take 111 us a call where a staged
+// copy, a flag and a kernel took 124 and a pitched copy 119.  Larger calls are copied as they
+// are and padded by a kernel, which also checks them above kHostCheckBytes (its answer
+// costs a copy back and a wait, about 11 us, which is what the host's pass over 64 KB costs
+// at most).  With a checking loop on the host and a pitched copy in its place, scoring
+// 1024 solutions of 8 x 1001 codons took 7.1 - 10.8 ms a call; now 0.76 ms.
+// staging: device space for all rows (L bytes each, rounded up to 16), or nullptr.
+constexpr size_t kHostCheckBytes = 64 * 1024, kHostRowBytes = 64 * 1024;
+static int upload_ids(pe_instance *in, TempBufs &t, const uint8_t *host, size_t rows, uint8_t *staging, uint8_t *ids)
 {
     const Shape &s = in->s;
-    const size_t bytes = rows * s.L;
-    unsigned long long bad = ~0ull;
+    const size_t L = (size_t)s.L, Lp = (size_t)s.Lp, bytes = rows * L;
+    int rc;
     if (bytes <= kHostCheckBytes) {
         uint64_t any = 0, v = 0;
         size_t i = 0;
@@ -1218,21 +1232,38 @@ static int upload_ids(pe_instance *in, const uint8_t *host, size_t rows, uint8_t
             any |= v;
         }
         for (; i < bytes; i++) any |= host[i];
-        if (any & 0xc0c0c0c0c0c0c0c0ull)
-            for (bad = 0; host[bad] < PE_NUM_CODON;) bad++;
-        d_bad = nullptr;
-    } else {
-        CK(cudaMemsetAsync(d_bad, 0xff, sizeof *d_bad, in->stream));
-    }
-    if (bad == ~0ull) {
-        CK(cudaMemcpyAsync(staging, host, bytes, cudaMemcpyHostToDevice, in->stream));
-        CK(launch_unpack_rows(staging, rows, s.L, s.Lp, ids, d_bad, in->stream));
-        if (d_bad) {
-            CK(cudaMemcpyAsync(&bad, d_bad, sizeof bad, cudaMemcpyDeviceToHost, in->stream));
-            CK(cudaStreamSynchronize(in->stream));
+        if (any & 0xc0c0c0c0c0c0c0c0ull) {
+            for (i = 0; host[i] < PE_NUM_CODON;) i++;
+            return fail(PE_ERR_ARG, "codon id out of range at %zu", i);
+        }
+        if (L == Lp || rows * Lp <= kHostRowBytes) {
+            const uint8_t *src = host;
+            if (L != Lp) {
+                uint8_t *padded;
+                if ((rc = t.host(&padded, rows * Lp))) return rc;
+                for (size_t r = 0; r < rows; r++) {
+                    memcpy(padded + r * Lp, host + r * L, L);
+                    memset(padded + r * Lp + L, 0, Lp - L);
+                }
+                src = padded;
+            }
+            CK(cudaMemcpyAsync(ids, src, rows * Lp, cudaMemcpyHostToDevice, in->stream));
+            return PE_OK;
         }
     }
-    if (bad != ~0ull) return fail(PE_ERR_ARG, "codon id out of range at %zu", (size_t)bad);
+    unsigned long long *d_bad = nullptr, bad = ~0ull;
+    if (bytes > kHostCheckBytes) {
+        if ((rc = t.get(&d_bad, 1))) return rc;
+        CK(cudaMemsetAsync(d_bad, 0xff, sizeof *d_bad, in->stream));
+    }
+    if (!staging && (rc = t.get(&staging, (bytes + 15) & ~size_t(15)))) return rc;
+    CK(cudaMemcpyAsync(staging, host, bytes, cudaMemcpyHostToDevice, in->stream));
+    CK(launch_unpack_rows(staging, rows, s.L, s.Lp, ids, d_bad, in->stream));
+    if (d_bad) {
+        CK(cudaMemcpyAsync(&bad, d_bad, sizeof bad, cudaMemcpyDeviceToHost, in->stream));
+        CK(cudaStreamSynchronize(in->stream));
+        if (bad != ~0ull) return fail(PE_ERR_ARG, "codon id out of range at %zu", (size_t)bad);
+    }
     return PE_OK;
 }
 
@@ -1249,12 +1280,7 @@ int pe_eval_objectives(pe_instance *in, const uint8_t *codon_idx, int32_t n, flo
     if ((rc = t.pop(s, b, n))) return rc;
     if ((rc = t.get(&part, (size_t)n * s.nres))) return rc;
     if ((rc = t.get(&counter, (size_t)n))) return rc;
-    uint8_t *staging;
-    unsigned long long *d_bad;
-    const size_t rows = (size_t)n * s.m;
-    if ((rc = t.get(&staging, (rows * s.L + 15) & ~size_t(15)))) return rc;
-    if ((rc = t.get(&d_bad, 1))) return rc;
-    if ((rc = upload_ids(in, codon_idx, rows, staging, b.ids, d_bad))) return rc;
+    if ((rc = upload_ids(in, t, codon_idx, (size_t)n * s.m, nullptr, b.ids))) return rc;
     CK(cudaMemsetAsync(b.obj, 0, (size_t)n * s.M * sizeof(float), in->stream));
     CK(cudaMemsetAsync(b.objidx, 0, (size_t)n * 2 * s.M, in->stream));
     CK(cudaMemsetAsync(counter, 0, (size_t)n * sizeof(int32_t), in->stream));
@@ -1287,10 +1313,8 @@ int pe_mutate(pe_instance *in, uint32_t generation, const int32_t *idx, int32_t 
     std::vector<int32_t> ident(n);
     for (int i = 0; i < n; i++) ident[i] = i;
     // staged in the children's ids, which the variation kernel writes later
-    unsigned long long *d_bad;
     const size_t rows = (size_t)n * s.m;
-    if ((rc = t.get(&d_bad, 1))) return rc;
-    if ((rc = upload_ids(in, parents, rows, dst.ids, src.ids, d_bad))) return rc;
+    if ((rc = upload_ids(in, t, parents, rows, dst.ids, src.ids))) return rc;
     CK(cudaMemcpyAsync(src.obj, pobj, (size_t)n * s.M * sizeof(float), cudaMemcpyHostToDevice, in->stream));
     CK(cudaMemcpyAsync(src.objidx, pobjidx, (size_t)n * 2 * s.M, cudaMemcpyHostToDevice, in->stream));
     CK(cudaMemcpyAsync(src.pql, ppql, (size_t)n * 3 * sizeof(int32_t), cudaMemcpyHostToDevice, in->stream));
@@ -1298,16 +1322,26 @@ int pe_mutate(pe_instance *in, uint32_t generation, const int32_t *idx, int32_t 
     CK(cudaMemcpyAsync(d_idx, idx, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, in->stream));
     CK(cudaMemcpyAsync(d_g, &generation, sizeof(uint32_t), cudaMemcpyHostToDevice, in->stream));
     CK(launch_mutate(s, in->d_tab, in->d_aa, src, dst, d_par, d_idx, n, -1, 0, d_g, d_ops, nullptr, in->stream));
-    if (children) {  // packed over the parents' ids, which nothing reads any more
+    // few children come back as padded rows, which the host strips; more are packed over the
+    // parents' ids, which nothing reads any more
+    uint8_t *padded = nullptr;
+    if (children) {
         const uint8_t *rows_out = dst.ids;
-        if (s.Lp != s.L) {
-            CK(launch_pack_rows(dst.ids, rows, s.L, s.Lp, src.ids, in->stream));
-            rows_out = src.ids;
+        if (s.Lp != s.L && rows * s.Lp <= kHostRowBytes) {
+            if ((rc = t.host(&padded, rows * s.Lp))) return rc;
+            CK(cudaMemcpyAsync(padded, dst.ids, rows * s.Lp, cudaMemcpyDeviceToHost, in->stream));
+        } else {
+            if (s.Lp != s.L) {
+                CK(launch_pack_rows(dst.ids, rows, s.L, s.Lp, src.ids, in->stream));
+                rows_out = src.ids;
+            }
+            CK(cudaMemcpyAsync(children, rows_out, rows * s.L, cudaMemcpyDeviceToHost, in->stream));
         }
-        CK(cudaMemcpyAsync(children, rows_out, rows * s.L, cudaMemcpyDeviceToHost, in->stream));
     }
     if (ops) CK(cudaMemcpyAsync(ops, d_ops, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, in->stream));
     CK(cudaStreamSynchronize(in->stream));
+    if (padded)
+        for (size_t r = 0; r < rows; r++) memcpy(children + r * s.L, padded + r * s.Lp, s.L);
     return PE_OK;
 }
 
