@@ -1217,8 +1217,9 @@ int pe_read_objectives_async(pe_instance *in, float *obj)
 // costs a copy back and a wait, about 11 us, which is what the host's pass over 64 KB costs
 // at most).  With a checking loop on the host and a pitched copy in its place, scoring
 // 1024 solutions of 8 x 1001 codons took 7.1 - 10.8 ms a call; now 0.76 ms.
-// staging: device space for all rows (L bytes each, rounded up to 16), or nullptr.
-constexpr size_t kHostCheckBytes = 64 * 1024, kHostRowBytes = 64 * 1024;
+// staging: device space for all rows (L bytes each, rounded up to 16), or nullptr: then the
+// rows pass through kStagingBytes at most, whatever their number.
+constexpr size_t kHostCheckBytes = 64 * 1024, kHostRowBytes = 64 * 1024, kStagingBytes = 16 << 20;
 static int upload_ids(pe_instance *in, TempBufs &t, const uint8_t *host, size_t rows, uint8_t *staging, uint8_t *ids)
 {
     const Shape &s = in->s;
@@ -1256,9 +1257,16 @@ static int upload_ids(pe_instance *in, TempBufs &t, const uint8_t *host, size_t 
         if ((rc = t.get(&d_bad, 1))) return rc;
         CK(cudaMemsetAsync(d_bad, 0xff, sizeof *d_bad, in->stream));
     }
-    if (!staging && (rc = t.get(&staging, (bytes + 15) & ~size_t(15)))) return rc;
-    CK(cudaMemcpyAsync(staging, host, bytes, cudaMemcpyHostToDevice, in->stream));
-    CK(launch_unpack_rows(staging, rows, s.L, s.Lp, ids, d_bad, in->stream));
+    size_t part = rows;  // rows copied at a time
+    if (!staging) {
+        part = std::min(rows, std::max<size_t>(1, kStagingBytes / L));
+        if ((rc = t.get(&staging, (part * L + 15) & ~size_t(15)))) return rc;
+    }
+    for (size_t r = 0; r < rows; r += part) {
+        const size_t k = std::min(part, rows - r);
+        CK(cudaMemcpyAsync(staging, host + r * L, k * L, cudaMemcpyHostToDevice, in->stream));
+        CK(launch_unpack_rows(staging, k, s.L, s.Lp, ids + r * Lp, d_bad, r * L, in->stream));
+    }
     if (d_bad) {
         CK(cudaMemcpyAsync(&bad, d_bad, sizeof bad, cudaMemcpyDeviceToHost, in->stream));
         CK(cudaStreamSynchronize(in->stream));

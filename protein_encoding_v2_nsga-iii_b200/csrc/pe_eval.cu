@@ -1076,9 +1076,9 @@ __device__ __forceinline__ uint4 shifted_piece(const uint4 *__restrict__ p, int 
 
 // packed: rows x L bytes, 16-byte aligned, readable up to the next multiple of 16;
 // ids: rows x Lp, zero past L.  *bad, where given, takes the index of the
-// first id >= 64.
+// first id >= 64, counted from base.
 __global__ void __launch_bounds__(256) k_unpack_rows(const uint8_t *__restrict__ packed, size_t rows, int L, int Lp,
-                                                     uint8_t *__restrict__ ids, unsigned long long *bad)
+                                                     uint8_t *__restrict__ ids, unsigned long long *bad, size_t base)
 {
     const int per = Lp >> 4;
     const size_t total = rows * per;
@@ -1097,7 +1097,7 @@ __global__ void __launch_bounds__(256) k_unpack_rows(const uint8_t *__restrict__
         if (bad && ((w[0] | w[1] | w[2] | w[3]) & 0xc0c0c0c0u)) {
             int k = 0;
             while (!((w[k >> 2] >> (8 * (k & 3))) & 0xc0u)) k++;
-            atomicMin(bad, (unsigned long long)(at + k));
+            atomicMin(bad, (unsigned long long)(base + at + k));
         }
         reinterpret_cast<uint4 *>(ids)[e] = make_uint4(w[0], w[1], w[2], w[3]);
     }
@@ -1132,10 +1132,10 @@ __global__ void __launch_bounds__(256) k_pack_rows(const uint8_t *__restrict__ i
 static int row_blocks(size_t pieces) { return (int)std::min<size_t>((pieces + 255) / 256, 148 * 16); }
 
 cudaError_t launch_unpack_rows(const uint8_t *packed, size_t rows, int L, int Lp, uint8_t *ids, unsigned long long *bad,
-                               cudaStream_t st)
+                               size_t base, cudaStream_t st)
 {
     if (rows == 0) return cudaSuccess;
-    k_unpack_rows<<<row_blocks(rows * (Lp >> 4)), 256, 0, st>>>(packed, rows, L, Lp, ids, bad);
+    k_unpack_rows<<<row_blocks(rows * (Lp >> 4)), 256, 0, st>>>(packed, rows, L, Lp, ids, bad, base);
     return cudaGetLastError();
 }
 

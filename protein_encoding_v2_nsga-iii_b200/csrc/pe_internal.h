@@ -162,10 +162,10 @@ cudaError_t launch_sl_queue(const SlJob *jobs, int njobs, int32_t *ticket, int n
 cudaError_t raise_smem_limit(const void *func, size_t bytes);
 size_t var_smem_bytes(const Shape &s);
 // codon ids from contiguous rows of L bytes (readable up to the next multiple of 16) to
-// rows of Lp, zero past L, *bad (preset to ~0; nullptr: unchecked) taking the index of the first id >= 64;
-// and back.  packed is 16-byte aligned.
+// rows of Lp, zero past L, *bad (preset to ~0; nullptr: unchecked) taking the index of the
+// first id >= 64, counted from `base`; and back.  packed is 16-byte aligned.
 cudaError_t launch_unpack_rows(const uint8_t *packed, size_t rows, int L, int Lp, uint8_t *ids, unsigned long long *bad,
-                               cudaStream_t st);
+                               size_t base, cudaStream_t st);
 cudaError_t launch_pack_rows(const uint8_t *ids, size_t rows, int L, int Lp, uint8_t *packed, cudaStream_t st);
 
 // records a message for pe_last_error() (pe_api.cu)

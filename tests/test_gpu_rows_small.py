@@ -40,3 +40,30 @@ def test_small_calls(pe, orc, gpu, L, m, n):
                 with pytest.raises(pe.PeError) as e:
                     call()
                 assert e.value.code == 1 and str(e.value).endswith(f"at {first}")
+
+
+def test_large_calls_stage_in_parts(pe, gpu):
+    """96 MB of ids pass through 16 MB of staging at a time: the scores of the parts taken
+    one by one, the first bad id of a later part, and no device memory for a second copy."""
+    import torch
+    L, m, n = 1000, 8, 12000
+    tabc = pe.dirichlet_table(L)
+    tab = tabc.arrays()
+    aa = pe.synthetic_protein(L - 1, L)
+    ids = rand_ids(np.random.default_rng(L), aa, tab, m, n)
+    with pe.Engine(aa, tabc, m, 8, 0.2, objectives=1, ref_p=2) as eng:
+        eng.evaluate(ids[:1])
+        before = torch.cuda.mem_get_info()[0]
+        whole = eng.evaluate(ids)
+        took = before - torch.cuda.mem_get_info()[0]     # the pool keeps what a call had at most
+        # the solutions themselves: ids in rows of 1008, bit planes (96 words of 8 bytes a CDS), results
+        own = n * m * (1008 + 96 * 8) + n * (16 + 8 + 12 + 8 * m + 4)
+        assert took < own + (48 << 20)
+        for k in range(0, n, 4000):
+            for a, b in zip(whole, eng.evaluate(ids[k:k + 4000])):
+                assert same(a[k:k + 4000], b)
+        first = (50 << 20) + 7
+        ids.reshape(-1)[[first, first + 1, ids.size - 1]] = 64
+        with pytest.raises(pe.PeError) as e:
+            eng.evaluate(ids)
+        assert str(e.value).endswith(f"at {first}")
