@@ -968,12 +968,19 @@ static cudaError_t launch_fronts_nadir(const Shape &s, const float *obj, float *
 // takes SOLS solutions, its lanes the points, and finds the largest s^2 (MM
 // multiply-adds a pair; a point read from shared memory serves the SOLS solutions);
 // a second pass over the points evaluates the reference's own formula, operation by
-// operation, for those whose s^2 comes within kAssocSlack * F of it.  Which points that
-// leaves cannot change the result: s^2 is off by less than 1e-6 F (MM products and the
-// rounded u), the reference's rounded squared distance by less than 2e-6 F (its
-// residuals are each off by at most (MM + 3) 2^-24 |f|), and equal distances after the
-// square root differ by less than 2.4e-7 of the squared ones; all together below a
-// third of the slack.  Where F is not inside 1e-30 .. 1e30 (overflow, subnormals,
+// operation, for those whose s^2 comes within kAssocSlack * F of it.  The others cannot
+// be nearest (e = 2^-24, first order, M = MM):
+//  - s^2 here is off by (3 M + 11) e F at most: |w|^2 by M roundings, halved by the
+//    reciprocal root, whose own error is 4 e, and one for u make u off by (M/2 + 5) e, the M
+//    multiply-adds add M e |f| to s, and squaring doubles both and rounds once;
+//  - the reference's squared distance by (M + 2.5) e F: the errors of its quotient move the
+//    residual along w, to which the residual is perpendicular (second order); rounding k w
+//    and the difference moves it by e (|s| + |residual|), which is 2.42 e F at most in
+//    the square, and the sum of squares takes M roundings;
+//  - distances equal after the square root differ by 4 e F at most in the square.
+// Two points each: a point of the reference's smallest distance has an s^2 within
+// (8 M + 31) e F of the largest one, 3.8e-6 F for four objectives and 4.8e-6 F for six; the
+// slack is four times that.  Where F is not inside 1e-30 .. 1e30 (overflow, subnormals,
 // infinities, NaN) every point is evaluated; a point of NaN s is too.
 // Measured: 36.8 us for 8192 solutions and 4060 points of four objectives (the whole
 // selection call 488 -> 471 us), 5.9 us for 2048 solutions and 165 points (was 6.8).
