@@ -269,9 +269,8 @@ cudaError_t mark(pe_instance *in, int k)
 }
 
 // the selection of a generation whose children sit in buf[dst]
-cudaError_t enqueue_selection(pe_instance *in, int dst, bool pdl_first)
+cudaError_t enqueue_selection(pe_instance *in, int dst)
 {
-    (void)pdl_first;
     return launch_select(in->s, in->buf[dst].obj, in->d_ext, in->d_ref, in->sc, in->d_surv, in->d_gen, 1, in->stream);
 }
 
@@ -290,8 +289,7 @@ cudaError_t enqueue_generation(pe_instance *in, int src)
     e = launch_sl(s, in->buf[dst], s.N, s.N, in->d_part, in->d_counter, in->d_status, in->stream, in->d_scanned, true);
     if (e != cudaSuccess) return e;
     if ((e = mark(in, 2)) != cudaSuccess) return e;
-    e = launch_select(s, in->buf[dst].obj, in->d_ext, in->d_ref, in->sc, in->d_surv, in->d_gen, 1, in->stream);
-    if (e != cudaSuccess) return e;
+    if ((e = enqueue_selection(in, dst)) != cudaSuccess) return e;
     return mark(in, 3);
 }
 
@@ -787,7 +785,7 @@ static int batch_capture(pe_batch *b, int gens, cudaGraphExec_t *out)
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->master, c.done, 0);
         }
         if (e == cudaSuccess)
-            e = batch_branches(b, [&](int i, pe_instance *in) { return enqueue_selection(in, 1 - src[i], false); });
+            e = batch_branches(b, [&](int i, pe_instance *in) { return enqueue_selection(in, 1 - src[i]); });
         for (int i = 0; i < n; i++) src[i] = 1 - src[i];
     }
     cudaError_t e2 = cudaStreamEndCapture(b->master, &g);
