@@ -80,13 +80,13 @@ L2_FLUSH_BYTES = 256 << 20
 # changes without a new capture.
 SL_NCU = {
     "hairpin": {"workload": "L=1000 m=8 N=1024, generation 1 (2311 CDSs scanned)",
-                "scans": 2311, "cells": 10389102811, "warp_inst": 31266309, "alu_warp_inst": 11443600,
-                "smem_wavefronts": 4298194, "thread_inst": 902909483, "dram_bytes": 2336000,
-                "issue_pct": 65.54, "alu_pct": 46.30, "smem_pct": 29.67, "source": "1d0658e3b7e05b61"},
+                "scans": 2311, "cells": 10389102811, "warp_inst": 31265971, "alu_warp_inst": 11443548,
+                "smem_wavefronts": 4298040, "thread_inst": 902927355, "dram_bytes": 2336000,
+                "issue_pct": 65.06, "alu_pct": 46.25, "smem_pct": 29.06, "source": "25cc877d1c68f614"},
     "lrcs": {"workload": "L=3000 m=4 N=4096, generation 1 (18320 CDS pairs scanned)",
-             "scans": 18320, "cells": 1250515745682, "warp_inst": 1225799901, "alu_warp_inst": 499049791,
-             "smem_wavefronts": 143171375, "thread_inst": 34777159841, "dram_bytes": 31119872,
-             "issue_pct": 44.77, "alu_pct": 36.31, "smem_pct": 20.58, "source": "1d0658e3b7e05b61"},
+             "scans": 18320, "cells": 1250515745682, "warp_inst": 1225808844, "alu_warp_inst": 499051202,
+             "smem_wavefronts": 143171051, "thread_inst": 34777241708, "dram_bytes": 31109888,
+             "issue_pct": 44.74, "alu_pct": 36.28, "smem_pct": 20.55, "source": "25cc877d1c68f614"},
 }
 SM_COUNT, ISSUE_WARP_INST_PER_SM_CLK, SMEM_WAVEFRONTS_PER_SM_CLK, ALU_WARP_INST_PER_SM_CLK = 148, 4, 1, 2
 # kernels one generation launches (one CUDA graph replay): k_variation, k_sl, k_dominance,

@@ -1841,7 +1841,9 @@ __device__ bool sl_seed_repetitive(const SlGeo &geo, const uint2 *__restrict__ S
     }
     if (lane == 0) atomicAdd(sum, (int)hits);
     __syncthreads();
-    return *sum > kSeedMostHits * kSeedBlocks;
+    const bool repetitive = *sum > kSeedMostHits * kSeedBlocks;
+    __syncthreads();  // the band scan clears the word before its first barrier
+    return repetitive;
 }
 
 // Returns false (CTA-uniform) when the CDS is too repetitive or some thread passed its
