@@ -935,8 +935,8 @@ __device__ __forceinline__ void front0_nadir(const Shape &s, const float *__rest
 // Front peeling (the first cluster) beside the nadir (one CTA; the rest of the second
 // cluster leaves at once).  Neither waits for the other, so the two take the time of
 // the longer one and one launch instead of their sum and two
-// (2048 solutions: 18.0 us, median over a run's first 60 generations, where the two
-// kernels took 13.5 and 10.4 on average; a design run of N = 128 6.91 -> 6.50 ms).
+// (2048 solutions: 18.0 us on average over a run's first 60 generations, where the two
+// kernels took 13.5 and 10.4; a design run of N = 128 6.91 -> 6.50 ms).
 template <int MM>
 __global__ void __cluster_dims__(kFrontCtas, 1, 1) __launch_bounds__(kFrontThreads, 1)
     k_fronts_nadir(Shape s, const float *__restrict__ obj, float *ext, SelectScratch sc)
