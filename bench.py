@@ -80,13 +80,13 @@ L2_FLUSH_BYTES = 256 << 20
 # changes without a new capture.
 SL_NCU = {
     "hairpin": {"workload": "L=1000 m=8 N=1024, generation 1 (2311 CDSs scanned)",
-                "scans": 2311, "cells": 10389102811, "warp_inst": 31265971, "alu_warp_inst": 11443548,
-                "smem_wavefronts": 4298040, "thread_inst": 902927355, "dram_bytes": 2336000,
-                "issue_pct": 65.06, "alu_pct": 46.25, "smem_pct": 29.06, "source": "25cc877d1c68f614"},
+                "scans": 2311, "cells": 10389102811, "warp_inst": 31265662, "alu_warp_inst": 11443469,
+                "smem_wavefronts": 4298309, "thread_inst": 902915700, "dram_bytes": 2335488,
+                "issue_pct": 65.44, "alu_pct": 46.24, "smem_pct": 29.39, "source": "404f96c82d72b477"},
     "lrcs": {"workload": "L=3000 m=4 N=4096, generation 1 (18320 CDS pairs scanned)",
-             "scans": 18320, "cells": 1250515745682, "warp_inst": 1225808844, "alu_warp_inst": 499051202,
-             "smem_wavefronts": 143171051, "thread_inst": 34777241708, "dram_bytes": 31109888,
-             "issue_pct": 44.74, "alu_pct": 36.28, "smem_pct": 20.55, "source": "25cc877d1c68f614"},
+             "scans": 18320, "cells": 1250515745682, "warp_inst": 1225802229, "alu_warp_inst": 499049872,
+             "smem_wavefronts": 143171340, "thread_inst": 34777519863, "dram_bytes": 31201280,
+             "issue_pct": 44.79, "alu_pct": 36.31, "smem_pct": 20.61, "source": "404f96c82d72b477"},
 }
 SM_COUNT, ISSUE_WARP_INST_PER_SM_CLK, SMEM_WAVEFRONTS_PER_SM_CLK, ALU_WARP_INST_PER_SM_CLK = 148, 4, 1, 2
 # kernels one generation launches (one CUDA graph replay): k_variation, k_sl, k_dominance,

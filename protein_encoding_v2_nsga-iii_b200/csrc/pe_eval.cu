@@ -1815,14 +1815,17 @@ __device__ __forceinline__ void seed_measure(uint32_t q, const SlGeo &geo, const
 // The sample costs less than 1 % of the band scan; with the bound alone repetitive LRCS
 // designs of 12603 to 27003 nucleotides took 1.8 - 4.4 times the band scan's time, now
 // 0.73 - 1.0.
+// A function of its own: as part of the scan it cost the scan's registers and schedule more
+// than its own time (design runs of 6 x 15003 nucleotides, 100 generations of 1024, mean of
+// two proteins timed twice: 96.3 ms inline, 94.9 called, 95.1 without sampling).
 // sum: one word of shared memory, cleared.
 constexpr int kSeedSamples = 1024, kSeedBlocks = 32, kSeedMostHits = 4;
 template <int NT, int FL>
-__device__ bool sl_seed_repetitive(const SlGeo &geo, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
+__device__ __noinline__ bool sl_seed_repetitive(int n, const uint2 *__restrict__ S, const uint32_t *__restrict__ Tlo,
                                    const uint32_t *__restrict__ Thi, uint32_t *heads, int nh, int *sum, int tid)
 {
     constexpr int K = Seed<FL>::K, t = Seed<FL>::step;
-    const int npos = geo.n - K + 1, nlook = (npos + t - 1) / t, lane = tid & 31, warp = tid >> 5;
+    const int npos = n - K + 1, nlook = (npos + t - 1) / t, lane = tid & 31, warp = tid >> 5;
 #pragma unroll 4
     for (int k = 0; k < kSeedSamples / NT; k++) {
         const int p = (int)__umulhi((uint32_t)(tid + k * NT) * 0x9E3779B1u, (uint32_t)npos), w = (p >> 5) + kSlGuardRows;
@@ -1866,7 +1869,7 @@ __device__ bool sl_seed_scan(const SlGeo &geo, const uint2 *__restrict__ S, cons
     const bool sampled = SAMPLED && n > kSeedSampleN;
     if (sampled && tid == 0) *sum = 0;
     __syncthreads();
-    if (sampled && sl_seed_repetitive<NT, FL>(geo, S, Tlo, Thi, heads, nh, sum, tid)) return false;
+    if (sampled && sl_seed_repetitive<NT, FL>(n, S, Tlo, Thi, heads, nh, sum, tid)) return false;
     // two positions per thread and step, so their exchanges are in flight together
     for (int i = tid; i < npos; i += 2 * nth) {
         const int i2 = i + nth;
